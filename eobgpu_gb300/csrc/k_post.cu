@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B, double 
     if (tid == 0) {
         w.row_off[B] = total;
         w.queue[1] = (unsigned long long)total;
+        *(unsigned long long *)w.partial = 0;  // k_modes counts its close rows here
     }
 }
 
@@ -146,37 +147,97 @@ __device__ __forceinline__ int find_segment(const long long *off, int B, long lo
     return lo;
 }
 
+// rows closer than this to a neighbour [M] keep the log-Gamma sums (mode_eval.h); the
+// fine pass steps by 0.05 and halves
+constexpr double kCloseRows = 0.04;
+
 struct ModeArgs {
     int K;
     int ells[kMaxModes], mms[kMaxModes];
+    ModeConst mc[kMaxModes];
     int imr;  // also r and p_r as series for the merger-ringdown attachment
 };
 
+// Rows closer than kCloseRows to a neighbour are listed (in the spline
+// scratch, which is free until the splines) for k_modes_close: the two
+// evaluations in one kernel cost the others their registers and half the
+// instruction cache (five modes, 4096 binaries, splines included: 5.8 ms
+// against 4.2 ms).  FP64 issue bounds both: five modes and the Hamiltonian
+// take 645 FP64 instructions a row in the closed form, 2427 by the sums on
+// every row (4096 binaries: 9.32 ms -> 2.49 + 0.56 ms; 1024 ragged binaries,
+// (2,2) alone: 0.77 -> 0.36 + 0.07 ms).
 __global__ void __launch_bounds__(128) k_modes(Ws w, int B, ModeArgs ma)
 {
     const long long R = (long long)w.queue[1];
     const size_t Rc = (size_t)w.L.Bc * (size_t)w.L.Lc;
+    long long *list = (long long *)w.cD;
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < R; r += (long long)gridDim.x * blockDim.x) {
         const int b = find_segment(w.row_off, B, r);
         const int i = (int)(r - w.row_off[b]);
         const BinaryRec &rec = w.bins[b];
         const double *row = w.traj + ((size_t)b * w.L.Lc + i) * kTrajStride;
         const double rr = row[1], phi = row[2], pr = row[3], pphi = row[4];
+        const bool close = (i > 0 && row[0] - row[-kTrajStride] < kCloseRows) ||
+                           (i + 1 < w.nsteps[b] && row[kTrajStride] - row[0] < kCloseRows);
         w.tin[r] = t_in_of(row[0], rec.Mt);
         w.ys[r] = phi;
         if (ma.imr) {
             w.imr_ys[r] = rr;
             w.imr_ys[Rc + r] = pr;
         }
+        if (close) {
+            list[atomicAdd((unsigned long long *)w.partial, 1ull)] = r;
+            continue;
+        }
+        HamEval e;
+        ham_eval(rec.ham, rr, pr, pphi, &e);
+        // v = omega^(1/3); v_phi = r (omega_c^2 r^3)^(-1/3) omega = omega omega_c^(-2/3)
+        const double ro = eob_rcbrt(e.dHdL), rc = eob_rcbrt(e.omega_c);
+        const ModeRow mr = mode_row(e.dHdL * (ro * ro), e.Hreal, e.dHdL * (rc * rc), pphi, rec.flux.inv2eta, phi);
+        for (int j = 0; j < ma.K; ++j) {
+            const int l = ma.ells[j], m = ma.mms[j];
+            const int li = lm_index(l, m);
+            const cdbl hl = mode_term(w.fac[b], l, m, ma.mc[j], mr, rec.pre_re[li], rec.pre_im[li], rec.nu, 0.0, true);
+            w.ys[(size_t)(1 + 2 * j) * Rc + r] = hl.re;
+            w.ys[(size_t)(2 + 2 * j) * Rc + r] = hl.im;
+        }
+    }
+}
+
+// The listed rows, by the log-Gamma sums: one thread per row, or per row and
+// mode while the list is short.
+__global__ void __launch_bounds__(128) k_modes_close(Ws w, int B, ModeArgs ma)
+{
+    // log l! for l = 0..8, summed as mode_eval_sums would
+    __shared__ double lfact[kLMax + 1];
+    if (threadIdx.x <= kLMax) {
+        double f = 0.0;
+        for (int q = 2; q <= (int)threadIdx.x; ++q) f += log((double)q);
+        lfact[threadIdx.x] = f;
+    }
+    __syncthreads();
+    const long long *list = (const long long *)w.cD;
+    const long long C = *(const long long *)w.partial, nt = (long long)gridDim.x * blockDim.x;
+    const size_t Rc = (size_t)w.L.Bc * (size_t)w.L.Lc;
+    const int per = (C * ma.K <= nt) ? 1 : ma.K, parts = ma.K / per;
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < C * parts; c += nt) {
+        const long long r = list[c % C];
+        const int j0 = (int)(c / C) * per;
+        const int b = find_segment(w.row_off, B, r);
+        const int i = (int)(r - w.row_off[b]);
+        const BinaryRec &rec = w.bins[b];
+        const double *row = w.traj + ((size_t)b * w.L.Lc + i) * kTrajStride;
+        const double rr = row[1], phi = row[2], pr = row[3], pphi = row[4];
         HamEval e;
         ham_eval(rec.ham, rr, pr, pphi, &e);
         const double v = cbrt(e.dHdL);
         const double vphi_in = 1.0 / (e.omega_c * e.omega_c * rr * rr * rr);
-        for (int j = 0; j < ma.K; ++j) {
+        const double Omega = v * v * v, vh = cbrt(e.Hreal * Omega), vPhi = rr * cbrt(vphi_in) * Omega;
+        for (int j = j0; j < j0 + per; ++j) {
             const int l = ma.ells[j], m = ma.mms[j];
             const int li = lm_index(l, m);
-            const cdbl hl = mode_eval(w.fac[b], l, m, rec.pre_re[li], rec.pre_im[li], rec.nu, rr, phi, pphi, v,
-                                      e.Hreal, vphi_in, 0.0, true);
+            const cdbl hl = mode_eval_sums(w.fac[b], l, m, rec.pre_re[li], rec.pre_im[li], rec.nu, phi, pphi, v, vh,
+                                           e.Hreal, vPhi, lfact[l], 0.0, true);
             w.ys[(size_t)(1 + 2 * j) * Rc + r] = hl.re;
             w.ys[(size_t)(2 + 2 * j) * Rc + r] = hl.im;
         }
@@ -503,8 +564,10 @@ cudaError_t launch_prepare_post(const Ws &w, const RunArgs &a, cudaStream_t s)
     ModeArgs ma;
     ma.K = a.K;
     for (int j = 0; j < kMaxModes; ++j) { ma.ells[j] = a.ells[j]; ma.mms[j] = a.mms[j]; }
+    for (int j = 0; j < a.K; ++j) ma.mc[j] = mode_const(a.ells[j], a.mms[j]);
     ma.imr = (a.opt.imr && w.imr_ys) ? 1 : 0;
     k_modes<<<nsm * 8, 128, 0, s>>>(w, a.B, ma);
+    k_modes_close<<<nsm * 4, 128, 0, s>>>(w, a.B, ma);
     const int nmain = 1 + 2 * a.K;
     const int nsubs = nmain + (ma.imr ? 2 : 0);
     // series per block: all of a binary's (its matrix is factorised once),

@@ -1,0 +1,81 @@
+"""Write trig_table.h: the tables of eob_sincos and of the Gamma phase.
+
+kSinQ[i] = RN(sin(2 pi i / 2048)), i = 0..512 (a quarter wave; the cosine is
+read backwards), and 2 pi / 2048 as the sum of two doubles.
+
+kArgGamma[l - 2][k]: coefficients, in z = (y / (l + 1))^2, of a polynomial for
+arg Gamma(l + 1 + i y) / y on 0 <= z <= 0.81, l = 2..8.  The function is
+analytic there (nearest singularity z = -1, the pole of Gamma at 0), so the
+Chebyshev interpolant of degree 19 is within 3e-17 of it, relative to its
+value; it is converted to powers of z at 60 digits.
+
+Values come from mpmath; the output is hexadecimal floating point, so the
+header is the same on every machine.
+
+    python gen_trig_table.py > trig_table.h
+"""
+import mpmath as mp
+
+mp.mp.dps = 60
+DEG, ZMAX = 19, mp.mpf("0.81")
+
+
+def arg_gamma_over_y(l, z):
+    y = mp.sqrt(z) * (l + 1)
+    if y < mp.mpf("1e-20"):
+        return mp.psi(0, l + 1)
+    return mp.im(mp.loggamma(mp.mpc(l + 1, y))) / y
+
+
+def fit(f, n, zmax, tol):
+    """Coefficients in powers of z of the Chebyshev interpolant of f on [0, zmax] at n nodes."""
+    nodes = [mp.cos(mp.pi * (2 * j + 1) / (2 * n)) for j in range(n)]
+    fv = [f((x + 1) / 2 * zmax) for x in nodes]
+    cheb = [mp.mpf(2 if k else 1) / n * sum(fv[j] * mp.cos(k * mp.pi * (2 * j + 1) / (2 * n)) for j in range(n))
+            for k in range(n)]
+    # Chebyshev series in x -> powers of x -> powers of z, x = 2 z / zmax - 1
+    t0, t1 = [mp.mpf(1)], [mp.mpf(0), mp.mpf(1)]
+    px = [mp.mpf(0)] * n
+    for k in range(n):
+        t = t0 if k == 0 else t1
+        for i, c in enumerate(t):
+            px[i] += cheb[k] * c
+        if k >= 1:
+            t2 = [mp.mpf(0)] + [2 * c for c in t1]
+            for i, c in enumerate(t0):
+                t2[i] -= c
+            t0, t1 = t1, t2
+    pz = [mp.mpf(0)] * n
+    for i, c in enumerate(px):  # c (2 z / zmax - 1)^i
+        for j in range(i + 1):
+            pz[j] += c * mp.binomial(i, j) * (2 / zmax) ** j * (-1) ** (i - j)
+    err = max(abs(mp.polyval(pz[::-1], z) / f(z) - 1) for z in [zmax * q / 200 for q in range(201)])
+    assert err < tol, err
+    return pz
+
+
+def coefficients(l):
+    return fit(lambda z: arg_gamma_over_y(l, z), DEG + 1, ZMAX, mp.mpf("3e-17"))
+
+
+def row(v, per=4):
+    v = [float(x).hex() for x in v]
+    return ",\n    ".join(", ".join(v[i:i + per]) for i in range(0, len(v), per))
+
+
+def main():
+    print("// Written by gen_trig_table.py: quarter-wave sine table and Gamma-phase polynomials.")
+    print("#pragma once")
+    step = 2 * mp.pi / 2048
+    hi = mp.mpf(float(step))
+    print(f"#define EOB_TRIG_STEP_HI {float(hi).hex()}")
+    print(f"#define EOB_TRIG_STEP_LO {float(step - hi).hex()}")
+    print(f"#define EOB_TRIG_INV {float(1 / step).hex()}")
+    print("#define EOB_SINQ_INIT { \\\n    " + row([mp.sin(step * i) for i in range(513)]).replace("\n", " \\\n") + "}")
+    rows = ["{" + row(coefficients(l)).replace("\n", " \\\n") + "}" for l in range(2, 9)]
+    print(f"#define EOB_ARG_GAMMA_N {DEG + 1}")
+    print(f"#define EOB_ARG_GAMMA_ZMAX {float(ZMAX)!r}")
+    print("#define EOB_ARG_GAMMA_INIT { \\\n    " + ", \\\n    ".join(rows) + "}")
+
+
+main()

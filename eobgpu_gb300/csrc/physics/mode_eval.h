@@ -4,17 +4,34 @@
 //   h_lm = T_lm e^{i delta_lm} S_lm (rho_lm^l + f_lm) h^N_lm,
 //   T_lm = Gamma(l + 1 - 2 i k) / l! e^{pi k} e^{2 i k log(4 m Omega / sqrt(e))},
 //   k = m H_real Omega,  h^N_lm = n_lm vPhi^(l+eps) Y_{l-eps}^{-m}(pi/2, phi).
-// The complex Gamma function is our own: an upward shift by the recurrence
-// Gamma(z) = Gamma(z + n) / prod_{j<n} (z + j) (Abramowitz & Stegun 6.1.15)
-// and the Stirling series for log Gamma (A&S 6.1.40) at Re(z + n) >= 16.
-// Only exp() of the log is ever used, so the branch of the complex logarithm
-// does not matter.  The reference's SciPy-derived loggamma is not used.
 //
+// Written for FP64 issue rate: what the modes of a row share (log v, powers,
+// S of either parity) is formed once (ModeRow), and T_lm has no logarithm or
+// arctangent of its own.  With y = 2 k,
+//   |Gamma(l + 1 - i y)|^2 e^{pi y} = prod_{j<=l} (j^2 + y^2) 2 pi y / (1 - e^{-2 pi y})
+// (A&S 6.1.31, the closed form of the flux), and arg Gamma(l + 1 - i y) =
+// -y P_l(y^2 / (l + 1)^2) with a polynomial per l (fasttrig.h) for
+// y <= 0.9 (l + 1), which every frequency of an inspiral meets (y < 2 m
+// Omega, Omega < 0.45).  Larger y go through the complex log Gamma: an
+// upward shift by the recurrence (A&S 6.1.15) and the Stirling series (A&S
+// 6.1.40) at Re(z) >= 16; only exp() of it is used, so the branch of its
+// logarithm does not matter.  The reference's SciPy-derived loggamma is not
+// used.
+//
+// mode_eval_sums is the evaluation by the sums of log Gamma throughout.  They
+// cancel from ~30 to order one and leave 4e-15 of rounding in the modulus
+// (rms against 40 digits; 1.5e-15 the closed form).  On rows closer than the
+// fine pass's step of 0.05 M (steps halved at the plunge) the third differences
+// of the spline amplify rounding by 1e7 and more, so that c3 there is rounding; k_modes keeps
+// those rows (3 in 100) on the sums, so that their tables do not move with the
+// evaluation of the others.
 // With derotate = true the result is multiplied by e^{i m phi}: the
 // e^{-i m phi} of the spherical harmonic is simply not applied, which is what
 // the spline inputs of the synthesis need (eob/seobnrv4phm.py:2331).
 #pragma once
 #include "fac_coeffs.h"
+#include "fasttrig.h"
+#include "flux_eval.h"
 
 namespace eob {
 
@@ -62,18 +79,18 @@ EOB_HD void cloggamma_shifted(double zr, double zi, double *lg_re, double *lg_im
     *lg_im = im;
 }
 
-// h_lm (or h_lm e^{i m phi} when derotate). i = lm_index(l, m).
-EOB_HD cdbl mode_eval(const FacCoeffs &fc, int l, int m, double pre_re, double pre_im, double eta, double r, double phi,
-                      double pphi, double v, double Hreal, double vPhiInput, double h22_calib, bool derotate)
+// h_lm (or h_lm e^{i m phi} when derotate) with T_lm from the sums of log Gamma, exp() and the
+// library's logarithms.  vh = (H_real v^3)^(1/3), lfact = log(l!), i = lm_index(l, m)
+EOB_HD cdbl mode_eval_sums(const FacCoeffs &fc, int l, int m, double pre_re, double pre_im, double eta, double phi,
+                           double pphi, double v, double vh, double Hreal, double vPhi, double lfact, double h22_calib,
+                           bool derotate)
 {
     if (eta > 0.25 && eta < 0.25 + 1e-4) eta = 0.25;
     const int i = lm_index(l, m);
     const double v2 = v * v;
     const double Omega = v2 * v;
     const double vh3 = Hreal * Omega;
-    const double vh = cbrt(vh3);
     const double eulerlog = kEulerGamma + log(2.0 * m * v);
-    const double vPhi = r * cbrt(vPhiInput) * Omega;
     const int eps = (l + m) % 2;
     // |Y| part and Newtonian amplitude: n_lm vPhi^(l+eps) (-1)^m Y_{l-eps}^m(pi/2, 0)
     double vpow = 1.0;
@@ -106,8 +123,6 @@ EOB_HD cdbl mode_eval(const FacCoeffs &fc, int l, int m, double pre_re, double p
     const double hk = Hreal * k;
     double lgr, lgi;
     cloggamma_shifted(l + 1.0, -2.0 * hk, &lgr, &lgi);
-    double lfact = 0.0;
-    for (int q = 2; q <= l; ++q) lfact += log((double)q);
     const double tmod = kPi * hk + lgr - lfact;
     double phase = 2.0 * hk * log(4.0 * k / 1.6487212707001281468) + lgi + delta;  // sqrt(e)
     if (!derotate) phase -= m * phi;
@@ -116,6 +131,123 @@ EOB_HD cdbl mode_eval(const FacCoeffs &fc, int l, int m, double pre_re, double p
     const double amp = exp(tmod) * S * vpow * y0;
     const cdbl e = {amp * cp, amp * sp};
     return cmul(cmul(e, rf), cdbl{pre_re, pre_im});
+}
+
+// What the modes of one trajectory point share.
+struct ModeRow {
+    double v, lv;       // omega^(1/3) and its logarithm
+    double Omega, Hreal;  // v^3, H_real
+    double vPhi;
+    double Se, So;      // source terms of even and odd l + m
+    double phi;
+};
+
+EOB_HD ModeRow mode_row(double v, double Hreal, double vPhi, double pphi, double inv2eta, double phi)
+{
+    ModeRow w;
+    w.v = v;
+    w.lv = eob_log(v);
+    w.Omega = v * v * v;
+    w.Hreal = Hreal;
+    w.vPhi = vPhi;
+    w.Se = fma(fma(Hreal, Hreal, -1.0), inv2eta, 1.0);
+    w.So = v * pphi;
+    w.phi = phi;
+    return w;
+}
+
+// What depends on (l, m) alone.
+struct ModeConst {
+    double elog;   // gamma + log(2 m)
+    double tail;   // log(4 m / sqrt(e))
+    double y0;     // (-1)^m Y_{l-eps}^m(pi/2, 0)
+    double ifact;  // 1 / l!
+};
+
+EOB_HD ModeConst mode_const(int l, int m)
+{
+    ModeConst c;
+    c.elog = kEulerGamma + log(2.0 * m);
+    c.tail = log(4.0 * m / 1.6487212707001281468);  // sqrt(e)
+    c.y0 = ((m % 2) ? -1.0 : 1.0) * ylm_equator(l - (l + m) % 2, m);
+    c.ifact = 1.0;
+    for (int q = 2; q <= l; ++q) c.ifact /= (double)q;
+    return c;
+}
+
+// h_lm (or h_lm e^{i m phi} when derotate). i = lm_index(l, m).
+EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, const ModeRow &w, double pre_re,
+                      double pre_im, double eta, double h22_calib, bool derotate)
+{
+    if (eta > 0.25 && eta < 0.25 + 1e-4) eta = 0.25;
+    const int i = lm_index(l, m);
+    const int eps = (l + m) % 2;
+    const double v = w.v, v2 = v * v, vh3 = w.Hreal * w.Omega;
+    // delta_lm: the builder assigns vh^3, vh^6, vh^9 and v^5 only
+    double delta = vh3 * fma(vh3, fma(vh3, fc.dvh[i][9], fc.dvh[i][6]), fc.dvh[i][3]);
+    delta = fma(fc.dv[i][5], v2 * v2 * v, delta);
+    // rho_lm^l + f_lm (rho up to v^10, eulerlog parts at v^6, v^8, v^10; f from v^1 and v^3..v^6, l <= 5)
+    const double el = mc.elog + w.lv;
+    double rho = fma(fc.rhol[i][10], el, fc.rho[i][10]);
+#pragma unroll
+    for (int k = 9; k >= 1; --k) {
+        double ck = fc.rho[i][k];
+        if (k == 6 || k == 8) ck = fma(fc.rhol[i][k], el, ck);
+        rho = fma(rho, v, ck);
+    }
+    rho = fma(rho, v, 1.0);
+    if (l == 2 && m == 2) {
+        const double v4 = v2 * v2;
+        rho = fma(h22_calib, v4 * v4 * v4, rho);
+    }
+    double rpl = rho;
+    for (int q = 1; q < l; ++q) rpl *= rho;
+    double fr = 0.0;
+    if (l <= 5) {
+        const double *f = fc.fre[i];
+        fr = v * fma(v2, fma(v, fma(v, fma(v, f[6], f[5]), f[4]), f[3]), f[1]);
+    }
+    const double fi = fc.fim_vh6[i] * vh3 * vh3;
+    cdbl rf = {rpl + fr, fi};
+    if (eta == 0.25 && (m % 2)) rf = {fr, fi};
+    // T_lm: its modulus and its phase without the logarithm's term
+    const double k = m * w.Omega, hk = w.Hreal * k, y = 2.0 * hk;
+    double tmod, targ;
+    const double q = y * (1.0 / (l + 1)), z = q * q;
+    if (y >= 0.0 && z <= EOB_ARG_GAMMA_ZMAX) {
+        targ = -y * arg_gamma_over_y(l, z);
+        const double y2 = y * y, x = 2.0 * kPi * y;
+        double p = 1.0;
+        for (int j = 1; j <= l; ++j) p *= y2 + (double)(j * j);
+#ifdef __CUDA_ARCH__
+        const double t2 = x * eob_rcp(-eob_expm1_neg(x)) * p;
+        tmod = t2 * eob_rsqrt(t2) * mc.ifact;
+#else
+        tmod = sqrt(x / -expm1(-x) * p) * mc.ifact;
+#endif
+    } else {
+        double lgr;
+        cloggamma_shifted(l + 1.0, -y, &lgr, &targ);
+        tmod = exp(kPi * hk + lgr) * mc.ifact;
+    }
+    double phase = fma(y, fma(3.0, w.lv, mc.tail), targ) + delta;
+    if (!derotate) phase -= m * w.phi;
+    double sp, cp;
+    eob_sincos(phase, &sp, &cp);
+    double vpow = 1.0;
+    for (int j = 0; j < l + eps; ++j) vpow *= w.vPhi;
+    const double amp = tmod * (eps ? w.So : w.Se) * vpow * mc.y0;
+    const cdbl e = {amp * cp, amp * sp};
+    return cmul(cmul(e, rf), cdbl{pre_re, pre_im});
+}
+
+// the same from the reference's arguments (vPhiInput = 1 / (omega_c^2 r^3))
+EOB_HD cdbl mode_eval(const FacCoeffs &fc, int l, int m, double pre_re, double pre_im, double eta, double r, double phi,
+                      double pphi, double v, double Hreal, double vPhiInput, double h22_calib, bool derotate)
+{
+    const double e4 = (eta > 0.25 && eta < 0.25 + 1e-4) ? 0.25 : eta;
+    const ModeRow w = mode_row(v, Hreal, r * cbrt(vPhiInput) * (v * v * v), pphi, 0.5 / e4, phi);
+    return mode_term(fc, l, m, mode_const(l, m), w, pre_re, pre_im, eta, h22_calib, derotate);
 }
 
 }  // namespace eob
