@@ -117,7 +117,7 @@ struct Ws {
     long long *row_off, *chunk_off;
     int *npts;
     double *tin, *ys, *cA, *cB, *cC, *cD, *partial;
-    float *f32;    // mixed precision: y, c1, c2, c3 of the mode series, [4][2K][rows]
+    float *f32;    // mixed precision: (y, c1, c2, c3) of the mode series, [2K][rows][4]
     float *dataf;  // mixed precision: data in FP32
     // merger-ringdown section (null when the workspace has none)
     double *imr_ys, *imr_cA, *imr_cB, *imr_cC, *imr_cD;  // series 0: r, 1: p_r

@@ -1,8 +1,8 @@
-// After the integrator: packing, multipoles on the trajectory, batched
-// not-a-knot splines, and the fused synthesis + likelihood pass.
+// After the integrator: packing, multipoles on the trajectory and batched
+// not-a-knot splines.
 //
-//  k_scan_*    one block: per-binary row counts and waveform sample counts,
-//              exclusive scans (packed ragged layout), sum of data^2.
+//  k_scan_rows one block: per-binary row counts and waveform sample counts,
+//              exclusive scan (packed ragged layout).
 //  k_modes     one thread per packed trajectory row: h_lm e^{i m phi} for the
 //              requested modes (get_hlms, eob/seobnrv4phm.py:2138-2221, and
 //              the de-rotation of compute_full_waveform, :2331).
@@ -10,18 +10,13 @@
 //              splines with the reference's tridiagonal set-up
 //              (src/interpolate.cu:10-267), the matrix factorised once per
 //              binary and solved by scans (spline_block.cuh).
-//  k_synth     one block per 1024-sample chunk of one binary: spline
-//              evaluation on the uniform grid (eob/seobnrv4phm.py:274-386,
-//              2310-2372), mode sum (BBHWaveformTD, :715-721) and the
-//              white-noise residual, reduced to one partial per chunk; in
-//              likelihood mode the strain is never written to memory.
-//  k_finalize  per binary, partials summed in a fixed order (deterministic).
+//
+// The synthesis and likelihood pass that follows is k_synth.cu.
 #include "eob_device.cuh"
+#include "packing.cuh"
 #include "spline_block.cuh"
 
 namespace eob {
-
-constexpr int kScanThreads = 1024;
 
 __device__ __forceinline__ double t_in_of(double t_M, double Mt)
 {
@@ -38,29 +33,10 @@ __device__ int binary_npts(const double *tr, int L, double Mt, double dt)
     return (int)((t1 - t0) / dT) + 1;
 }
 
-// block-wide exclusive scan helper: returns the exclusive prefix of v over the block
-template <int NT>
-__device__ long long block_exclusive_scan(long long v, long long *sm, long long *total)
-{
-    const int tid = threadIdx.x;
-    sm[tid] = v;
-    __syncthreads();
-    for (int off = 1; off < NT; off <<= 1) {
-        const long long add = (tid >= off) ? sm[tid - off] : 0;
-        __syncthreads();
-        sm[tid] += add;
-        __syncthreads();
-    }
-    const long long incl = sm[tid];
-    if (total) *total = sm[NT - 1];
-    __syncthreads();
-    return incl - v;
-}
-
 // rows and uniform-grid sample counts per binary; packed row offsets
 __global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B, double dt)
 {
-    __shared__ long long sm[kScanThreads];
+    __shared__ long long sm[34];
     const int tid = threadIdx.x;
     const int per = (B + kScanThreads - 1) / kScanThreads;
     const int b0 = tid * per;
@@ -91,60 +67,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B, double 
         w.queue[1] = (unsigned long long)total;
         *(unsigned long long *)w.partial = 0;  // k_modes counts its close rows here
     }
-}
-
-// synthesis work items: chunks of kChunk samples of min(npts, N) samples per
-// binary (all N samples when cover_all); sum of data^2
-__global__ void __launch_bounds__(kScanThreads) k_scan_chunks(Ws w, int B, int N, int cover_all, const double *data,
-                                                               int mixed)
-{
-    __shared__ long long sm[kScanThreads];
-    __shared__ double s_sq[kScanThreads];
-    const int tid = threadIdx.x;
-    const int per = (B + kScanThreads - 1) / kScanThreads;
-    const int b0 = tid * per;
-    const int b1 = min(B, b0 + per);
-    long long chunks = 0;
-    for (int b = b0; b < b1; ++b) {
-        const int np = w.npts[b];
-        const int nuse = (np <= 0) ? 0 : (cover_all ? N : (np < N ? np : N));
-        chunks += (nuse + kChunk - 1) / kChunk;
-    }
-    double sq = 0.0;
-    if (data)
-        for (int k = tid; k < N; k += kScanThreads) {
-            sq += data[k] * data[k];
-            if (mixed) w.dataf[k] = (float)data[k];
-        }
-    s_sq[tid] = sq;
-    long long total;
-    long long co = block_exclusive_scan<kScanThreads>(chunks, sm, &total);
-    for (int b = b0; b < b1; ++b) {
-        w.chunk_off[b] = co;
-        const int np = w.npts[b];
-        const int nuse = (np <= 0) ? 0 : (cover_all ? N : (np < N ? np : N));
-        co += (nuse + kChunk - 1) / kChunk;
-    }
-    for (int off = kScanThreads / 2; off > 0; off >>= 1) {
-        if (tid < off) s_sq[tid] += s_sq[tid + off];
-        __syncthreads();
-    }
-    if (tid == 0) {
-        w.chunk_off[B] = total;
-        w.queue[2] = (unsigned long long)total;
-        w.queue[3] = (unsigned long long)__double_as_longlong(s_sq[0]);
-    }
-}
-
-// index b with off[b] <= v < off[b+1]
-__device__ __forceinline__ int find_segment(const long long *off, int B, long long v)
-{
-    int lo = 0, hi = B;  // answer in [lo, hi)
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (off[mid] <= v) lo = mid; else hi = mid;
-    }
-    return lo;
 }
 
 // rows closer than this to a neighbour [M] keep the log-Gamma sums (mode_eval.h); the
@@ -271,12 +193,8 @@ struct PackedSplines {
         f.c3[i] = c3;
         if (mixed && s >= 1 && s < nmain) {
             // FP32 copies of the amplitude series for the mixed-precision synthesis
-            const size_t S = (size_t)2 * w.L.Kc * Rc;
-            float *q = w.f32 + (size_t)(s - 1) * Rc + base + i;
-            q[0] = (float)f.y[i];
-            q[S] = (float)c1;
-            q[2 * S] = (float)c2;
-            q[3 * S] = (float)c3;
+            reinterpret_cast<float4 *>(w.f32)[(size_t)(s - 1) * Rc + base + i] =
+                make_float4((float)f.y[i], (float)c1, (float)c2, (float)c3);
         }
     }
     __device__ void put_last(int b, int s, int i, const SplineSeries &f, double, double, double) const
@@ -307,254 +225,6 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline(Ws w, const int *orde
     PackedBlock::run(acc, sm, s0, min(nsubs, s0 + per));
 }
 
-struct SynthArgs {
-    int B, N, K;
-    int mms[kMaxModes];
-    double dt, amp;
-    const double *data;   // lnL mode
-    double *out;          // strain modes
-    int mode;             // 0: lnL, 1: summed strain (zero past the end), 2: per mode, t clamped to the end
-};
-
-// interval i with x[i] <= t < x[i+1] (searchsorted right - 1), t, x >= 0:
-// integer comparison of the IEEE bit patterns keeps the FP64 pipe free.
-__device__ __forceinline__ int knot_index(const double *x, int n, double t)
-{
-    const long long tb = __double_as_longlong(t);
-    int lo = 0, hi = n;  // first index with x > t lies in [lo, hi]
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__double_as_longlong(x[mid]) <= tb) lo = mid + 1; else hi = mid;
-    }
-    int i = lo - 1;
-    if (i < 0) i = 0;
-    if (i > n - 1) i = n - 1;
-    return i;
-}
-
-// the merger-ringdown of one mode x = t - t_match after the match point
-// (compute_MR_mode_free, eob/seobnrv4phm.py:1830-1843)
-__device__ __forceinline__ void ringdown_mode(const ImrRec &c, double x, double *hr, double *hi)
-{
-    const double A = c.c1c * tanh(c.c1f * x + c.c2f) + c.c2c;
-    const double ph = c.phi_match - c.d1c * log((1 + c.d2f * exp(-c.d1f * x)) / (1 + c.d2f)) - c.om_re * x;
-    const double mag = c.eta * A * exp(-c.om_im * x);
-    double sp, cp;
-    sincos(ph, &sp, &cp);
-    *hr = mag * cp;
-    *hi = mag * sp;
-}
-
-__global__ void __launch_bounds__(256) k_synth(Ws w, SynthArgs sa)
-{
-    __shared__ double s_red[256 / 32];
-    const long long C = (long long)w.queue[2];
-    const size_t Rc = (size_t)w.L.Bc * (size_t)w.L.Lc;
-    for (long long c = blockIdx.x; c < C; c += gridDim.x) {
-        const int b = find_segment(w.chunk_off, sa.B, c);
-        const int j = (int)(c - w.chunk_off[b]);
-        const int np = w.npts[b];
-        // with the merger-ringdown: samples 0 .. idx are the NQC-corrected
-        // inspiral, idx + 1 .. np - 1 the ringdown, zero beyond (per mode too)
-        const bool imr = w.imr_bin && w.imr_bin[b].on;
-        const int idx = imr ? w.imr_bin[b].idx : np;
-        const int nuse = (sa.mode == 2) ? sa.N : (np < sa.N ? np : sa.N);
-        const int n = w.nsteps[b];
-        const size_t base = (size_t)w.row_off[b];
-        const double *x = w.tin + base;
-        const double Mts = w.bins[b].Mt * kMTSUN_SI;
-        const double dT = sa.dt / Mts;
-        const double t0 = x[0], tend = x[n - 1];
-        const ImrRec *recs = imr ? w.imr_rec + (size_t)b * w.L.Kc : nullptr;
-        double acc = 0.0;
-        const int kbeg = j * kChunk;
-        const int kend = min(nuse, kbeg + kChunk);
-        for (int k = kbeg + threadIdx.x; k < kend; k += blockDim.x) {
-            double hsum = 0.0, hsum_i = 0.0;
-            if (imr && k > idx) {
-                if (k < np) {
-                    const double xr = (k - idx) * dT;
-                    for (int q = 0; q < sa.K; ++q) {
-                        double hr, hi;
-                        ringdown_mode(recs[q], xr, &hr, &hi);
-                        if (sa.mode == 2) {
-                            const size_t oo = 2 * (((size_t)b * sa.K + q) * (size_t)sa.N + k);
-                            sa.out[oo] = hr;
-                            sa.out[oo + 1] = hi;
-                        }
-                        hsum += hr;
-                        hsum_i += hi;
-                    }
-                } else if (sa.mode == 2) {
-                    for (int q = 0; q < sa.K; ++q) {
-                        const size_t oo = 2 * (((size_t)b * sa.K + q) * (size_t)sa.N + k);
-                        sa.out[oo] = 0.0;
-                        sa.out[oo + 1] = 0.0;
-                    }
-                }
-                if (sa.mode == 1) {
-                    sa.out[2 * ((size_t)b * sa.N + k)] = hsum;
-                    sa.out[2 * ((size_t)b * sa.N + k) + 1] = hsum_i;
-                } else if (sa.mode == 0) {
-                    const double hk = sa.amp * hsum;
-                    acc += hk * hk - 2.0 * sa.data[k] * hk;
-                }
-                continue;
-            }
-            double t = k * dT + t0;
-            if (t > tend) t = tend;
-            const int i = knot_index(x, n, t);
-            const double xx = t - x[i], x2 = xx * xx, x3 = x2 * xx;
-            const size_t o = base + i;
-            const double phi = w.ys[o] + w.cA[o] * xx + w.cB[o] * x2 + w.cC[o] * x3;
-            double rr = 0.0, pr = 0.0, om = 0.0;
-            if (imr) {
-                om = w.cA[o] + 2 * w.cB[o] * xx + 3 * w.cC[o] * x2;
-                rr = w.imr_ys[o] + w.imr_cA[o] * xx + w.imr_cB[o] * x2 + w.imr_cC[o] * x3;
-                const size_t op = Rc + o;
-                pr = w.imr_ys[op] + w.imr_cA[op] * xx + w.imr_cB[op] * x2 + w.imr_cC[op] * x3;
-            }
-            for (int q = 0; q < sa.K; ++q) {
-                const size_t orr = (size_t)(1 + 2 * q) * Rc + o, oi = (size_t)(2 + 2 * q) * Rc + o;
-                const double re = w.ys[orr] + w.cA[orr] * xx + w.cB[orr] * x2 + w.cC[orr] * x3;
-                const double im = w.ys[oi] + w.cA[oi] * xx + w.cB[oi] * x2 + w.cC[oi] * x3;
-                double sp, cp;
-                sincos(sa.mms[q] * phi, &sp, &cp);
-                // (re + i im) e^{-i m phi}
-                double hr = re * cp + im * sp, hi = im * cp - re * sp;
-                if (imr) {
-                    // NQC correction (EOBNonQCCorrection, eob/seobnrv4phm.py:1686-1700)
-                    const ImrRec &cq = recs[q];
-                    const double sr = sqrt(rr), rO = rr * om;
-                    const double mag = 1.0 + (pr * pr / (rO * rO)) * (cq.a1 + cq.a2 / rr + cq.a3 / (rr * sr));
-                    const double nph = cq.b1 * pr / rO + pr * pr * pr / rO * cq.b2;
-                    double ns, nc;
-                    sincos(nph, &ns, &nc);
-                    const double tr = mag * (hr * nc - hi * ns);
-                    hi = mag * (hr * ns + hi * nc);
-                    hr = tr;
-                }
-                if (sa.mode == 2) {
-                    const size_t oo = 2 * (((size_t)b * sa.K + q) * (size_t)sa.N + k);
-                    sa.out[oo] = hr;
-                    sa.out[oo + 1] = hi;
-                }
-                hsum += hr;
-                hsum_i += hi;
-            }
-            if (sa.mode == 1) {
-                sa.out[2 * ((size_t)b * sa.N + k)] = hsum;
-                sa.out[2 * ((size_t)b * sa.N + k) + 1] = hsum_i;
-            } else if (sa.mode == 0) {
-                const double hk = sa.amp * hsum;
-                acc += hk * hk - 2.0 * sa.data[k] * hk;
-            }
-        }
-        // block reduction (fixed order)
-        for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0 && sa.mode == 0) {
-            double s = 0.0;
-            for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += s_red[q];
-            w.partial[c] = s;
-        }
-        __syncthreads();
-    }
-}
-
-// Mixed precision synthesis: the phase spline and its reduction mod 2 pi run
-// in FP64; the amplitude splines (FP32 coefficient copies written at spline
-// build), sin/cos and the residual run in FP32.  mode 0 accumulates the lnL
-// terms with a Kahan-compensated FP32 sum per thread and FP64 chunk partials;
-// mode 1 writes the summed strain (zero past each waveform's end).  The
-// FP32 copies exist only if the spline build ran with precision 1 (workspace
-// flag queue[6]); otherwise the lnL comes out NaN.
-__global__ void __launch_bounds__(256) k_synth_mixed(Ws w, SynthArgs sa)
-{
-    __shared__ double s_red[256 / 32];
-    const long long C = (long long)w.queue[2];
-    const bool have_f32 = w.queue[6] == 1ull;
-    const size_t Rc = (size_t)w.L.Bc * (size_t)w.L.Lc;
-    const size_t S = (size_t)2 * w.L.Kc * Rc;
-    const double two_pi_hi = 6.283185307179586232, two_pi_lo = 2.4492935982947064e-16;
-    for (long long c = blockIdx.x; c < C; c += gridDim.x) {
-        const int b = find_segment(w.chunk_off, sa.B, c);
-        const int j = (int)(c - w.chunk_off[b]);
-        const int np = w.npts[b];
-        const int nuse = np < sa.N ? np : sa.N;
-        // the merger-ringdown runs in the FP64 synthesis only
-        const bool imr_bin = w.imr_bin && w.imr_bin[b].on;
-        const int n = w.nsteps[b];
-        const size_t base = (size_t)w.row_off[b];
-        const double *x = w.tin + base;
-        const double Mts = w.bins[b].Mt * kMTSUN_SI;
-        const double dT = sa.dt / Mts;
-        const double t0 = x[0], tend = x[n - 1];
-        float acc = 0.0f, comp = 0.0f;
-        const int kbeg = j * kChunk;
-        const int kend = have_f32 ? min(nuse, kbeg + kChunk) : kbeg;
-        for (int k = kbeg + threadIdx.x; k < kend; k += blockDim.x) {
-            double t = k * dT + t0;
-            if (t > tend) t = tend;
-            const int i = knot_index(x, n, t);
-            const double xx = t - x[i];
-            const size_t o = base + i;
-            const double phi = w.ys[o] + xx * (w.cA[o] + xx * (w.cB[o] + xx * w.cC[o]));
-            const float xf = (float)xx;
-            float h = 0.0f, hi = 0.0f;
-            for (int q = 0; q < sa.K; ++q) {
-                const size_t orr = (size_t)(2 * q) * Rc + o, oi = (size_t)(2 * q + 1) * Rc + o;
-                const float re = w.f32[orr] + xf * (w.f32[S + orr] + xf * (w.f32[2 * S + orr] + xf * w.f32[3 * S + orr]));
-                const float im = w.f32[oi] + xf * (w.f32[S + oi] + xf * (w.f32[2 * S + oi] + xf * w.f32[3 * S + oi]));
-                const double ph = sa.mms[q] * phi;
-                const double nn = rint(ph * 0.15915494309189533577);
-                const double red = fma(-nn, two_pi_lo, fma(-nn, two_pi_hi, ph));
-                float sp, cp;
-                sincosf((float)red, &sp, &cp);
-                // (re + i im) e^{-i m phi}
-                h = fmaf(re, cp, fmaf(im, sp, h));
-                hi = fmaf(im, cp, fmaf(-re, sp, hi));
-            }
-            if (sa.mode == 1) {
-                sa.out[2 * ((size_t)b * sa.N + k)] = (double)h;
-                sa.out[2 * ((size_t)b * sa.N + k) + 1] = (double)hi;
-            } else {
-                const float hk = (float)sa.amp * h;
-                const float term = hk * (hk - 2.0f * w.dataf[k]);
-                // Kahan summation
-                const float yv = term - comp;
-                const float tv = acc + yv;
-                comp = (tv - acc) - yv;
-                acc = tv;
-            }
-        }
-        double dacc = (double)acc - (double)comp;
-        for (int off = 16; off > 0; off >>= 1) dacc += __shfl_down_sync(0xffffffffu, dacc, off);
-        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = dacc;
-        __syncthreads();
-        if (threadIdx.x == 0 && sa.mode == 0) {
-            double sum = 0.0;
-            for (int q = 0; q < (int)(blockDim.x >> 5); ++q) sum += s_red[q];
-            w.partial[c] = (have_f32 && !imr_bin) ? sum : __longlong_as_double(0x7ff8000000000000ll);
-        }
-        __syncthreads();
-    }
-}
-
-__global__ void k_finalize(Ws w, int B, double *lnl, int *status_out)
-{
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const double dsq = __longlong_as_double((long long)w.queue[3]);
-    const int st = w.status[b];
-    double s = 0.0;
-    for (long long c = w.chunk_off[b]; c < w.chunk_off[b + 1]; ++c) s += w.partial[c];
-    const bool bad = (w.npts[b] <= 0);
-    if (lnl) lnl[b] = bad ? __longlong_as_double(0x7ff8000000000000LL) : -0.5 * (dsq + s);
-    if (status_out) status_out[b] = st;
-}
-
 cudaError_t launch_prepare_post(const Ws &w, const RunArgs &a, cudaStream_t s)
 {
     int dev = 0, nsm = 0;
@@ -579,34 +249,6 @@ cudaError_t launch_prepare_post(const Ws &w, const RunArgs &a, cudaStream_t s)
     }
     k_spline<<<dim3(a.B, (nsubs + per - 1) / per), kSplineThreads, 0, s>>>(w, a.order, nsubs, nmain, per,
                                                                           a.opt.precision == 1 ? 1 : 0);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_synth(const Ws &w, const RunArgs &a, int mode, double *out, cudaStream_t s)
-{
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int mixed = (mode != 2 && a.opt.precision == 1 && !a.opt.imr) ? 1 : 0;
-    k_scan_chunks<<<1, kScanThreads, 0, s>>>(w, a.B, a.N, mode == 2 ? 1 : 0, mode == 0 ? a.data : nullptr,
-                                             mode == 0 ? mixed : 0);
-    if (mode == 1) {
-        cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * 2 * (size_t)a.B * a.N, s);
-        if (e != cudaSuccess) return e;
-    }
-    SynthArgs sa;
-    sa.B = a.B;
-    sa.N = a.N;
-    sa.K = a.K;
-    for (int j = 0; j < kMaxModes; ++j) sa.mms[j] = a.mms[j];
-    sa.dt = a.dt;
-    sa.amp = a.amp;
-    sa.data = a.data;
-    sa.out = out;
-    sa.mode = mode;
-    if (mixed) k_synth_mixed<<<nsm * 8, 256, 0, s>>>(w, sa);
-    else k_synth<<<nsm * 8, 256, 0, s>>>(w, sa);
-    k_finalize<<<(a.B + 127) / 128, 128, 0, s>>>(w, a.B, mode == 0 ? a.lnl : nullptr, a.status_out);
     return cudaGetLastError();
 }
 

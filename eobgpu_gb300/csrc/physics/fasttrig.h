@@ -27,7 +27,12 @@ static constexpr double kArgGammaH[7][EOB_ARG_GAMMA_N] = EOB_ARG_GAMMA_INIT;
 
 #ifdef __CUDACC__
 // the rare arguments, out of line
-static __device__ __noinline__ void eob_sincos_large(double x, double *s, double *c) { sincos(x, s, c); }
+static __device__ __noinline__ double2 eob_sincos_large(double x)
+{
+    double2 r;
+    sincos(x, &r.x, &r.y);
+    return r;
+}
 #endif
 
 EOB_HD void eob_sincos(double x, double *s, double *c)
@@ -36,7 +41,9 @@ EOB_HD void eob_sincos(double x, double *s, double *c)
     constexpr double kShift = 6755399441055744.0;  // 1.5 2^52
     const unsigned xe = (unsigned)__double2hiint(x) & 0x7fffffffu;
     if (xe >= 0x42700000u) {  // |x| >= 2^40, inf, NaN
-        eob_sincos_large(x, s, c);
+        const double2 r = eob_sincos_large(x);
+        *s = r.x;
+        *c = r.y;
         return;
     }
     const double t = fma(x, EOB_TRIG_INV, kShift);
