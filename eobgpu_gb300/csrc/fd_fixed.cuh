@@ -1,0 +1,193 @@
+// The frequency-domain residual of one (bin, detector) on the integer units.
+//
+// |d - (F+ h+ + Fx hx) e^{-2 pi i f tau}|^2 / S takes 17 to 24 FP64 instructions,
+// and GB300 issues one in 64 cycles per SM sub-partition; a 32 x 32 + 64 bit
+// product takes 4.  Here the projection, the rotation and the difference are block
+// floating point: 64-bit integers with one exponent per vector (57 bits and
+// more where a double has 53), and the FP64 pipe keeps the
+// square and its weight: 3 instructions per (bin, detector), beside about 60 integer
+// products and shifts that issue meanwhile.
+//
+//  * dot_hi: a sum of two 64-bit products' upper halves from six 32-bit ones (the
+//    products of the low halves, below the last place, left out).
+//  * The delay phase is exact: f tau in units of 2^-64 turn is an integer product;
+//    sine and cosine come from a table in units of 2^-61, and the next bin of a
+//    thread by a rotation (2^-58 a step).
+//    A vector's components share an exponent, so a residual of exactly equal
+//    terms is 2^-57 of their size rather than zero.
+//  * The residual becomes a double again with its exponent, so weights, sums,
+//    infinite PSDs and the range are FP64's own.  Infinities, NaN and values above
+//    2^960 take the FP64 expression, one bin at a time; subnormals count as zero
+//    (their square is).
+#pragma once
+#include "eob_device.cuh"
+
+namespace eob {
+
+typedef long long i64;
+typedef unsigned long long u64;
+
+__device__ const i64 kSinFix[513] = EOB_SINFIX_INIT;
+constexpr int kFixTop = 1023 + 960;  // largest exponent field of the integer path
+
+// (a b + c d) / 2^64 for |a|, |c| <= 2^61 and |b|, |d| <= 2^61 (one unit low at most)
+__device__ __forceinline__ i64 dot_hi(i64 a, i64 b, i64 c, i64 d)
+{
+    const int ah = (int)(a >> 32), bh = (int)(b >> 32), ch = (int)(c >> 32), dh = (int)(d >> 32);
+    const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
+    const int cl = (int)((unsigned)c >> 1), dl = (int)((unsigned)d >> 1);
+    const i64 p = (i64)ah * bh + (i64)ch * dh;
+    const i64 q = (i64)ah * bl + (i64)al * bh + ((i64)ch * dl + (i64)cl * dh);
+    return p + (q >> 31);
+}
+
+__device__ __forceinline__ i64 mul_hi(i64 a, i64 b)
+{
+    const int ah = (int)(a >> 32), bh = (int)(b >> 32);
+    const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
+    return (i64)ah * bh + (((i64)ah * bl + (i64)al * bh) >> 31);
+}
+
+// u cycles per bin in units of 2^-64 turn (mod 1): an integer whose multiples
+// are the phases of the bins (turn_ok: |u| < 2^10)
+__device__ __forceinline__ bool turn_ok(double u)
+{
+    return (unsigned)(__double2hiint(u) & 0x7fffffff) < 0x40900000u;
+}
+
+__device__ __forceinline__ u64 turn_of(double u)
+{
+    const i64 b = __double_as_longlong(u);
+    const int e = (int)((b >> 52) & 0x7ff);
+    const u64 m = ((u64)b & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
+    const int sh = e - 1023 - 52 + 64;  // u = m 2^(e - 1023 - 52)
+    const u64 t = sh >= 0 ? (sh < 64 ? m << sh : 0ull) : (sh > -64 ? m >> -sh : 0ull);
+    return b < 0 ? 0ull - t : t;
+}
+
+// sin and cos of 2 pi t / 2^64 in units of 2^-61 (fasttrig.h's method)
+__device__ __forceinline__ void sincos_fix(u64 t, i64 *s, i64 *c)
+{
+    const u64 v = t + (1ull << 52);
+    const unsigned k = (unsigned)(v >> 53);
+    const i64 rem = (i64)(v & ((1ull << 53) - 1)) - (1ll << 52);
+    const i64 r = __mul64hi(rem << 9, 0x6487ed5110b4611all);  // 2 pi 2^60: the remainder, units of 2^-69
+    const u64 z = (u64)__mul64hi(r, r);                       // r^2, units of 2^-74
+    const unsigned zt = (unsigned)(z >> 24);
+    const unsigned z2 = __umulhi(zt, zt);                     // r^4, units of 2^-68
+    // cos r - 1 = -r^2 / 2 + r^4 / 24 and (sin r - r) / r = -r^2 / 6 + r^4 / 120, units of 2^-74
+    const i64 c1 = (i64)(((u64)z2 * 2863311531u) >> 30) - (i64)(z >> 1);
+    const i64 w = (i64)(((u64)z2 * 2290649225u) >> 32) - (i64)__umul64hi(z, 3074457345618258603ull);
+    const i64 sr = r + (__mul64hi(r, w << 8) >> 18);
+    const int i = k & 511;
+    const i64 st = __ldg(&kSinFix[i]), ct = __ldg(&kSinFix[512 - i]);
+    const i64 sv = st + (__mul64hi(ct, sr) >> 5) + (__mul64hi(st, c1) >> 10);
+    const i64 cv = ct - (__mul64hi(st, sr) >> 5) + (__mul64hi(ct, c1) >> 10);
+    const i64 sa = (k & 512) ? cv : sv, ca = (k & 512) ? sv : cv;
+    *s = (k & 1024) ? -sa : sa;
+    *c = ((k + 512) & 1024) ? -ca : ca;
+}
+
+// (c, s) turned by (rc, rs)
+__device__ __forceinline__ void rotate(i64 *s, i64 *c, i64 rs, i64 rc)
+{
+    const i64 cn = dot_hi(*c, rc, -*s, rs) << 3;
+    *s = dot_hi(*s, rc, *c, rs) << 3;
+    *c = cn;
+}
+
+__device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// x in units of 2^(e - 1023 - 52 - up) for an exponent field e >= that of x: |result| < 2^(53 + up)
+__device__ __forceinline__ i64 fix_of(double x, int e, int up)
+{
+    const i64 b = __double_as_longlong(x);
+    const int f = (int)((b >> 52) & 0x7ff);
+    const u64 m = (u64)((b & 0xfffffffffffffll) | 0x10000000000000ll) << up;
+    const u64 v = m >> min(e - f, 63);
+    return f == 0 ? 0 : (b < 0 ? -(i64)v : (i64)v);
+}
+
+// |v| 2^u as a double (rounded to nearest; zero below the normal range)
+__device__ __forceinline__ double size_of(i64 v, int u)
+{
+    const u64 a = (u64)(v < 0 ? -v : v);
+    const int z = __clzll((i64)a);
+    const u64 m = a << (z & 63);
+    const int e = 1023 + u + 63 - z;
+    // the mantissa's leading one carries into the exponent field, and so does a rounding up
+    const u64 b = ((u64)(unsigned)(e - 1) << 52) + (m >> 11) + ((m >> 10) & 1);
+    return __longlong_as_double((a == 0 || e < 1) ? 0ll : (i64)b);
+}
+
+// One (bin, detector) of the data: in units of 2^e, |.| < 2^57, and 1 / S (32 bytes).
+struct __align__(16) FdData {
+    i64 re, im;
+    double w;
+    int e, slow;
+};
+
+__device__ __forceinline__ FdData fd_data(double2 d, double S)
+{
+    const int f = max(exponent_of(d.x), exponent_of(d.y));
+    return {fix_of(d.x, f, 4), fix_of(d.y, f, 4), 1.0 / S, f - 1023 - 52 - 4, f > kFixTop};
+}
+
+// What the residual needs of a (binary, detector): the patterns in units of
+// 2^e, the phase per bin and its rotation over `stride` bins.
+struct FdDetector {
+    i64 fp, fx, rs, rc;
+    u64 step;
+    int e, slow;
+};
+
+__device__ __forceinline__ FdDetector fd_detector(double fp, double fx, double cycles_per_bin, int stride)
+{
+    FdDetector q;
+    const int e = max(exponent_of(fp), exponent_of(fx));
+    q.slow = !turn_ok(cycles_per_bin) || e > 1023 + 20 || (e < 1023 - 60 && e > 0);
+    q.fp = fix_of(fp, e, 8);
+    q.fx = fix_of(fx, e, 8);
+    q.e = e - 1023 - 60;
+    q.step = turn_of(cycles_per_bin);
+    sincos_fix(q.step * (u64)stride, &q.rs, &q.rc);
+    return q;
+}
+
+// The polarisations of one bin in units of 2^e, |.| < 2^60
+struct FdStrain {
+    i64 pr, pi, xr, xi;
+    int e;
+    bool slow;
+};
+
+__device__ __forceinline__ FdStrain fd_strain(double2 p, double2 x)
+{
+    const int e = max(max(exponent_of(p.x), exponent_of(p.y)), max(exponent_of(x.x), exponent_of(x.y)));
+    return {fix_of(p.x, e, 7), fix_of(p.y, e, 7), fix_of(x.x, e, 7), fix_of(x.y, e, 7), e - 1023 - 59, e > kFixTop};
+}
+
+// |d - (F+ h+ + Fx hx) (c - i s)|^2
+__device__ __forceinline__ double fd_power(const FdStrain &h, const FdDetector &q, i64 s, i64 c, const FdData &d)
+{
+    // the projection, |.| < 2^60, in units of 2^(h.e + q.e + 62); rotated, |.| < 2^58, of 2^(h.e + q.e + 65)
+    const i64 gr = dot_hi(h.pr, q.fp, h.xr, q.fx) << 2, gi = dot_hi(h.pi, q.fp, h.xi, q.fx) << 2;
+    const i64 tr = dot_hi(gr, c, gi, s), ti = dot_hi(gi, c, -gr, s);
+    const int et = h.e + q.e + 65;
+    const int u = max(et, d.e), st = min(u - et, 63), sd = min(u - d.e, 63);
+    const double rr = size_of((d.re >> sd) - (tr >> st), u), ri = size_of((d.im >> sd) - (ti >> st), u);
+    return fma(rr, rr, ri * ri);
+}
+
+// the same in FP64, for what the integers do not take
+static __device__ __noinline__ double fd_power_slow(double2 hp, double2 hx, double fp, double fx, double2 d,
+                                                    double cycles)
+{
+    double s, c;
+    sincos(2.0 * kPi * cycles, &s, &c);
+    const double gr = fma(fp, hp.x, fx * hx.x), gi = fma(fp, hp.y, fx * hx.y);
+    const double rr = d.x - fma(gr, c, gi * s), ri = d.y - fma(gi, c, -gr * s);
+    return fma(rr, rr, ri * ri);
+}
+
+}  // namespace eob

@@ -12,13 +12,17 @@
 // on the fly -- the bins f < N/2 + 1 read H(f) from the lower half and
 // H(N - f) from the mirrored block of the upper half, so every element of H
 // is read once and h~_+, h~_x are never written -- then projects onto every
-// detector and accumulates the residual.  The PSD enters as its reciprocal,
+// detector and accumulates the residual, on the integer units up to its square
+// (fd_fixed.cuh).  The PSD enters as its reciprocal,
 // formed once per call (a division costs about six FP64 issue slots on GB300,
 // a product one).  A last kernel sums each binary's block partials in a fixed
 // order (deterministic, no atomics).
 #include "eob_device.cuh"
+#include "fd_fixed.cuh"
 
 namespace {
+
+using namespace eob;
 
 constexpr int kFdThreads = 256;
 constexpr int kFdPerThread = 16;                      // bins per thread, kFdThreads apart
@@ -89,71 +93,72 @@ __global__ void k_detector_response(const double *ra, const double *dec, const d
     }
 }
 
-// 1 / S_n for every (detector, bin)
-__global__ void k_fd_inv_psd(const double *psd, long long n, double *ipsd)
+// data and 1 / S_n of every (detector, bin)
+__global__ void k_fd_data(const double2 *data, const double *psd, long long n, FdData *out)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        ipsd[i] = 1.0 / psd[i];
+        out[i] = fd_data(data[i], psd[i]);
+}
+
+// the (detector, binary) constants; the patterns are halved: the residual
+// takes twice the polarisations
+__global__ void k_fd_detectors(const double *Fplus, const double *Fcross, const double *tshift, double df, int n,
+                               FdDetector *det)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        det[i] = fd_detector(0.5 * Fplus[i], 0.5 * Fcross[i], df * tshift[i], kFdThreads);
 }
 
 // One block of kFdBins bins (f = df i, i < Nf = N / 2 + 1) of one binary:
 // sum over the NCH detectors of |d - (F+ h~_+ + Fx h~_x) e^{-2 pi i f tau}|^2
 // / S_n, h~ zero below start_ind.  partial[blockIdx.x * B + b].  Each thread
-// takes kFdPerThread bins kFdThreads apart; the delay phase comes from one
-// sincos at its first bin and one for the step, then rotations (a sincos
-// costs tens of FP64 instructions).  NCH is a template argument so that the
-// per-detector values stay in registers.
+// takes kFdPerThread bins kFdThreads apart.  NCH is a template argument so that
+// the per-detector values stay in registers.  Integer issue bounds it (60 % of all slots,
+// most of them half rate; the FP64 pipe 53 % busy): 512 binaries x 32769 bins x 3
+// detectors 2.25 ms in FP64 (84 % of its slots) -> 0.67 ms.  In pairs of floats (48 bits)
+// it was 0.47 ms, with five times the error.
 template <int NCH>
-__global__ void __launch_bounds__(kFdThreads) k_fd_split_lnl(const double2 *H, int N, int start_ind,
-                                                             const double2 *data, const double *ipsd,
-                                                             const double *Fplus, const double *Fcross,
-                                                             const double *tshift, double df, int B, double *partial)
+__global__ void __launch_bounds__(kFdThreads, NCH <= 3 ? 3 : 2) k_fd_split_lnl(
+    const double2 *H, int N, int start_ind, const double2 *data, const FdData *fixed, const FdDetector *det,
+    const double *Fplus, const double *Fcross, const double *tshift, double df, int B, double *partial)
 {
     __shared__ double warp_sum[kFdThreads / 32];
+    __shared__ FdDetector dets[NCH];
     const int Nf = N / 2 + 1;
     for (int b = blockIdx.y; b < B; b += gridDim.y) {
         const double2 *Hb = H + (size_t)b * N;
-        double fp[NCH], fx[NCH], s[NCH], co[NCH], sd[NCH], cd[NCH];
+        i64 s[NCH], co[NCH];
         const int i0 = blockIdx.x * kFdBins + threadIdx.x;
+        if (threadIdx.x < NCH) dets[threadIdx.x] = det[(size_t)threadIdx.x * B + b];
+        __syncthreads();
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-            fp[c] = Fplus[(size_t)c * B + b];
-            fx[c] = Fcross[(size_t)c * B + b];
-            const double tau = tshift[(size_t)c * B + b];
-            sincos(kTwoPi * (df * i0) * tau, &s[c], &co[c]);
-            sincos(kTwoPi * (df * kFdThreads) * tau, &sd[c], &cd[c]);
-        }
+        for (int c = 0; c < NCH; ++c) sincos_fix((u64)i0 * dets[c].step, &s[c], &co[c]);
         double acc = 0.0;
-#pragma unroll 4
         for (int q = 0; q < kFdPerThread; ++q) {
             const int i = i0 + q * kFdThreads;
-            if (q > 0) {
-#pragma unroll
-                for (int c = 0; c < NCH; ++c) {
-                    const double cn = fma(co[c], cd[c], -s[c] * sd[c]);
-                    s[c] = fma(s[c], cd[c], co[c] * sd[c]);
-                    co[c] = cn;
-                }
+            if (i >= Nf) break;
+            double2 p = make_double2(0.0, 0.0), x = p;
+            if (i >= start_ind) {
+                const double2 a = Hb[i];
+                const double2 z = Hb[i == 0 ? 0 : N - i];
+                // 2 h~_+ = a + conj z, 2 h~_x = (a - conj z) / i
+                p = make_double2(a.x + z.x, a.y - z.y);
+                x = make_double2(a.y + z.y, z.x - a.x);
             }
-            if (i < Nf) {
-                double pr = 0.0, pi = 0.0, xr = 0.0, xi = 0.0;
-                if (i >= start_ind) {
-                    const double2 a = Hb[i];
-                    const double2 z = Hb[i == 0 ? 0 : N - i];
-                    // h~_+ = (a + conj z) / 2, h~_x = (a - conj z) / 2i
-                    pr = 0.5 * (a.x + z.x);
-                    pi = 0.5 * (a.y - z.y);
-                    xr = 0.5 * (a.y + z.y);
-                    xi = -0.5 * (a.x - z.x);
-                }
+            const FdStrain h = fd_strain(p, x);
 #pragma unroll
-                for (int c = 0; c < NCH; ++c) {
-                    const double gr = fma(fp[c], pr, fx[c] * xr), gi = fma(fp[c], pi, fx[c] * xi);
-                    const double2 d = data[(size_t)c * Nf + i];
-                    const double rr = d.x - fma(gr, co[c], gi * s[c]);
-                    const double ri = d.y - fma(gi, co[c], -gr * s[c]);
-                    acc = fma(fma(rr, rr, ri * ri), ipsd[(size_t)c * Nf + i], acc);
+            for (int c = 0; c < NCH; ++c) {
+                if (q > 0) rotate(&s[c], &co[c], dets[c].rs, dets[c].rc);
+                const FdData d = fixed[(size_t)c * Nf + i];
+                double power;
+                if (h.slow || dets[c].slow || d.slow) {
+                    const size_t k = (size_t)c * B + b;
+                    power = fd_power_slow(p, x, 0.5 * Fplus[k], 0.5 * Fcross[k], data[(size_t)c * Nf + i],
+                                          df * i * tshift[k]);
+                } else {
+                    power = fd_power(h, dets[c], s[c], co[c], d);
                 }
+                acc = fma(power, d.w, acc);
             }
         }
 #pragma unroll
@@ -202,14 +207,14 @@ int eob_detector_response(const double *ra, const double *dec, const double *psi
     return cudaGetLastError() == cudaSuccess ? EOB_OK : EOB_E_CUDA;
 }
 
-// block partials of every binary, then 1 / S_n for up to kFdMaxChannels
-// detectors (256-byte aligned)
+// block partials of every binary, then the data with 1 / S_n and the per-binary
+// constants of up to kFdMaxChannels detectors (256-byte aligned)
 size_t eob_fd_lnl_scratch_bytes(int B, int N)
 {
     if (B < 1 || N < 2) return 0;
     const long long nblk = ((long long)(N / 2 + 1) + kFdBins - 1) / kFdBins;
     const size_t part = ((size_t)(nblk * B) * sizeof(double) + 255) & ~(size_t)255;
-    return part + (size_t)kFdMaxChannels * (size_t)(N / 2 + 1) * sizeof(double);
+    return part + (size_t)kFdMaxChannels * ((size_t)(N / 2 + 1) * sizeof(FdData) + (size_t)B * sizeof(FdDetector));
 }
 
 int eob_fd_lnl_from_fft(const double *H, int N, int start_ind, const double *data, const double *psd,
@@ -222,16 +227,19 @@ int eob_fd_lnl_from_fft(const double *H, int N, int start_ind, const double *dat
     const int nblk = (N / 2 + 1 + kFdBins - 1) / kFdBins;
     double *partial = (double *)scratch;
     const size_t part = ((size_t)nblk * (size_t)B * sizeof(double) + 255) & ~(size_t)255;
-    double *ipsd = (double *)((char *)scratch + part);
-    const long long npsd = (long long)nch * (N / 2 + 1);
-    k_fd_inv_psd<<<blocks_for(npsd, 256), 256, 0, stream>>>(psd, npsd, ipsd);
+    FdData *fixed = (FdData *)((char *)scratch + part);
+    const long long nbin = (long long)nch * (N / 2 + 1);
+    k_fd_data<<<blocks_for(nbin, 128), 128, 0, stream>>>((const double2 *)data, psd, nbin, fixed);
+    if (cudaGetLastError() != cudaSuccess) return EOB_E_CUDA;
+    FdDetector *det = (FdDetector *)(fixed + nbin);
+    k_fd_detectors<<<blocks_for((long long)nch * B, 64), 64, 0, stream>>>(Fplus, Fcross, time_shift, df, nch * B, det);
     if (cudaGetLastError() != cudaSuccess) return EOB_E_CUDA;
     dim3 grid(nblk, B < 65535 ? B : 65535);
     const double2 *H2 = (const double2 *)H, *d2 = (const double2 *)data;
 #define EOB_FD_LAUNCH(K)                                                                                         \
     case K:                                                                                                      \
-        k_fd_split_lnl<K><<<grid, kFdThreads, 0, stream>>>(H2, N, start_ind, d2, ipsd, Fplus, Fcross, time_shift, \
-                                                           df, B, partial);                                      \
+        k_fd_split_lnl<K><<<grid, kFdThreads, 0, stream>>>(H2, N, start_ind, d2, fixed, det, Fplus, Fcross,      \
+                                                           time_shift, df, B, partial);                          \
         break;
     switch (nch) {
         EOB_FD_LAUNCH(1) EOB_FD_LAUNCH(2) EOB_FD_LAUNCH(3) EOB_FD_LAUNCH(4)

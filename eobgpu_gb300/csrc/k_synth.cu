@@ -98,10 +98,18 @@ __device__ __forceinline__ int knot_index(const double *x, int lo, int hi, doubl
     return lo;
 }
 
+// k >= 0 as a double, by integer operations (a conversion takes an FP64 issue slot)
+__device__ __forceinline__ double index_value(int k)
+{
+    const int z = __clz(k);
+    const unsigned long long m = (unsigned long long)(unsigned)k << (z + 21) & 0xfffffffffffffull;
+    return k ? __longlong_as_double((long long)(m | ((unsigned long long)(1023 + 31 - z) << 52))) : 0.0;
+}
+
 // t_k = k dT + t0, at most tend (compared on the bits)
 __device__ __forceinline__ double grid_time(int k, double dT, double t0, double tend)
 {
-    const double t = fma((double)k, dT, t0);
+    const double t = fma(index_value(k), dT, t0);
     return __double_as_longlong(t) > __double_as_longlong(tend) ? tend : t;
 }
 
@@ -218,12 +226,15 @@ __device__ __forceinline__ void spline_sample(const Ws &w, const SynthArgs &sa, 
     const double phi = cubic(w.ys, w.cA, w.cB, w.cC, o, xx);
     double h = 0.0, hi = 0.0;
     if (!recs && sa.K > 1) {
-        double s1, c1, pc = 1.0, ps = 0.0;
+        double s1, c1;
         eob_sincos(phi, &s1, &c1);
+        double pc = c1, ps = s1;
         for (int m = 1; m <= sa.mmax; ++m) {
-            const double cn = fma(pc, c1, -(ps * s1));
-            ps = fma(ps, c1, pc * s1);
-            pc = cn;
+            if (m > 1) {
+                const double cn = fma(pc, c1, -(ps * s1));
+                ps = fma(ps, c1, pc * s1);
+                pc = cn;
+            }
             for (int q = 0; q < sa.K; ++q) {
                 if (sa.mms[q] != m) continue;
                 const double re = cubic(w.ys, w.cA, w.cB, w.cC, (size_t)(1 + 2 * q) * Rc + o, xx);
@@ -414,7 +425,8 @@ __device__ __forceinline__ void mixed_sample(const Ws &w, const SynthArgs &sa, s
         const double u = phi * 0.15915494309189533577;
         turn = (unsigned long long)__double_as_longlong(u - rint(u) + 98304.0);
     }
-    const float xf = (float)xx;
+    // to nearest (ties away): the truncated bits and the next one
+    const float xf = __uint_as_float(__float_as_uint(f32_trunc(xx)) + (((unsigned)__double2loint(xx) >> 28) & 1u));
     float h = 0.0f, hi = 0.0f;
     for (int q = 0; q < sa.K; ++q) {
         const float4 a = f32[(size_t)(2 * q) * Rc + o], c = f32[(size_t)(2 * q + 1) * Rc + o];

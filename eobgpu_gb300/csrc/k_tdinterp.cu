@@ -15,9 +15,10 @@
 // are clamped into the binary's rows (the reference reads whatever memory an
 // out-of-range index points at).  Complex
 // arrays are interleaved (re, im) doubles.  All three are grid-stride
-// streaming kernels: one thread per output sample (per frequency bin for the
-// likelihood, four bins per thread), coalesced over samples.
+// streaming kernels: one thread per output sample (four frequency bins for the
+// likelihood), coalesced over samples.
 #include "eob_device.cuh"
+#include "fd_fixed.cuh"
 
 namespace {
 
@@ -26,51 +27,54 @@ constexpr int kSumBins = 1024;   // frequency bins per likelihood partial (NUM_T
 constexpr int kSumThreads = 256;
 
 __device__ __forceinline__ double cubic(const double *y, const double *c1, const double *c2, const double *c3, size_t j,
-                                        double x, double x2, double x3)
+                                        double x)
 {
-    return y[j] + c1[j] * x + c2[j] * x2 + c3[j] * x3;
+    return fma(fma(fma(c3[j], x, c2[j]), x, c1[j]), x, y[j]);
 }
 
 // sum_k (re_k + i im_k) e^{-i m_k phi} of one sample; sub-series k of a
-// binary's block start at base + k * stride.  One mode: sincos(m phi) as the
-// reference.  Several modes: e^{i q phi} for q = 1 .. max m by complex
-// products of e^{i phi} (one FP64 sincos per sample instead of one per mode;
-// the powers agree with direct evaluation to ~q ulp), each mode taken at its
-// own q; modes with m outside 1..8 use their own sincos.
+// binary's block start at base + k * stride.  e^{i q phi} for q = 1 .. max m
+// by complex products of e^{i phi} (one sincos of 11 FP64 instructions per
+// sample, fasttrig.h; the powers agree with direct evaluation to ~q ulp), each
+// mode taken at its own q; modes with m outside 1..8 use their own sincos.
+// FP64 issue bounds it: two modes take 42 FP64 instructions a sample, 72 with
+// the library's sincos and products for the powers of x.
 __device__ __forceinline__ double2 mode_sum(const double *y, const double *c1, const double *c2, const double *c3,
                                             size_t base, size_t stride, int ind, double x, int K, const int *ms,
                                             int mmax)
 {
-    const double x2 = x * x, x3 = x * x2;
-    const double phi = cubic(y, c1, c2, c3, base + 2 * (size_t)K * stride + ind, x, x2, x3);
+    const double phi = cubic(y, c1, c2, c3, base + 2 * (size_t)K * stride + ind, x);
     double hr = 0.0, hi = 0.0;
     auto add = [&](int k, double c, double s) {
-        const double re = cubic(y, c1, c2, c3, base + (size_t)k * stride + ind, x, x2, x3);
-        const double im = cubic(y, c1, c2, c3, base + (size_t)(K + k) * stride + ind, x, x2, x3);
+        const double re = cubic(y, c1, c2, c3, base + (size_t)k * stride + ind, x);
+        const double im = cubic(y, c1, c2, c3, base + (size_t)(K + k) * stride + ind, x);
         // (re + i im)(c - i s)
-        hr += re * c + im * s;
-        hi += im * c - re * s;
+        hr = fma(re, c, fma(im, s, hr));
+        hi = fma(im, c, fma(-re, s, hi));
     };
     if (K == 1) {
         double s, c;
-        sincos(ms[0] * phi, &s, &c);
+        eob::eob_sincos(ms[0] * phi, &s, &c);
         add(0, c, s);
         return make_double2(hr, hi);
     }
-    double s1, cp1;
-    sincos(phi, &s1, &cp1);
-    double pc = 1.0, ps = 0.0;
-    for (int q = 1; q <= mmax; ++q) {
-        const double cn = pc * cp1 - ps * s1;
-        ps = fma(ps, cp1, pc * s1);
-        pc = cn;
-        for (int k = 0; k < K; ++k)
-            if (ms[k] == q) add(k, pc, ps);
+    if (mmax > 0) {
+        double s1, cp1;
+        eob::eob_sincos(phi, &s1, &cp1);
+        double pc = cp1, ps = s1;
+        for (int q = 1;; ++q) {
+            for (int k = 0; k < K; ++k)
+                if (ms[k] == q) add(k, pc, ps);
+            if (q == mmax) break;
+            const double cn = fma(pc, cp1, -(ps * s1));
+            ps = fma(ps, cp1, pc * s1);
+            pc = cn;
+        }
     }
     for (int k = 0; k < K; ++k) {
         if (ms[k] < 1 || ms[k] > 8) {
             double s, c;
-            sincos(ms[k] * phi, &s, &c);
+            eob::eob_sincos(ms[k] * phi, &s, &c);
             add(k, c, s);
         }
     }
@@ -126,55 +130,84 @@ __global__ void k_td1(double2 *out, const double *dataTime, const double *ts, co
     }
 }
 
-// |d - h|^2 / S_n summed over one block of kSumBins frequencies for one
-// (binary, channel): blockIdx.x = frequency block, y = binary, z = channel
-__global__ void __launch_bounds__(kSumThreads) k_fd_lnl(double2 *temp_sum, const double2 *hp, const double2 *hc,
-                                                        const double2 *data, const double *psd, const double *Fplus,
-                                                        const double *Fcross, const double *tshift, double df, int B,
-                                                        int nch, int N)
+// |d - h|^2 / S_n summed over blocks of kSumBins frequencies, per (binary,
+// channel): blockIdx.x = frequency block, y = group of binaries, z = pair of
+// channels.  The residual up to its square on the integer units (fd_fixed.cuh); a
+// block keeps its data and 1 / S_n in registers (four bins and NCH channels
+// per thread) and carries `group` binaries past them.  96 binaries x 30721 bins x 2
+// channels: 0.39 ms in FP64 -> 0.13 ms.
+constexpr int kSumGroup = 16;  // most binaries per block
+
+template <int NCH>
+__global__ void __launch_bounds__(kSumThreads, 2) k_fd_lnl(double2 *temp_sum, const double2 *hp, const double2 *hc,
+                                                           const double2 *data, const double *psd, const double *Fplus,
+                                                           const double *Fcross, const double *tshift, double df, int B,
+                                                           int group, int ch0, int nch, int N)
 {
-    __shared__ double warp_sum[kSumThreads / 32];
-    for (int b = blockIdx.y; b < B; b += gridDim.y) {
-        for (int ch = blockIdx.z; ch < nch; ch += gridDim.z) {
-            const double fp = Fplus[(size_t)ch * B + b], fc = Fcross[(size_t)ch * B + b];
-            const double tau = tshift[(size_t)ch * B + b];
-            // the thread's bins are kSumThreads apart: e^{-2 pi i f tau} at the
-            // first one, then rotations by e^{-2 pi i df kSumThreads tau}
-            const int i0 = blockIdx.x * kSumBins + threadIdx.x;
-            double s, co, sd, cd;
-            sincos(2.0 * eob::kPi * (df * i0) * tau, &s, &co);
-            sincos(2.0 * eob::kPi * (df * kSumThreads) * tau, &sd, &cd);
-            double acc = 0.0;
+    using namespace eob;
+    constexpr int kBins = kSumBins / kSumThreads, kWarps = kSumThreads / 32;
+    __shared__ FdDetector det[kSumGroup][NCH];
+    __shared__ double sums[kSumGroup][NCH][kWarps];
+    const int tid = threadIdx.x, i0 = blockIdx.x * kSumBins + tid, first = ch0 + blockIdx.z * NCH;
+    FdData d[kBins][NCH];
 #pragma unroll
-            for (int q = 0; q < kSumBins / kSumThreads; ++q) {
+    for (int q = 0; q < kBins; ++q)
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            const size_t at = (size_t)(first + c) * N + min(i0 + q * kSumThreads, N - 1);
+            d[q][c] = fd_data(data[at], psd[at]);
+        }
+    for (int b0 = blockIdx.y * group; b0 < B; b0 += gridDim.y * group) {
+        const int nb = min(group, B - b0);
+        __syncthreads();
+        for (int t = tid; t < nb * NCH; t += kSumThreads) {
+            const size_t k = (size_t)(first + t % NCH) * B + b0 + t / NCH;
+            det[t / NCH][t % NCH] = fd_detector(Fplus[k], Fcross[k], df * tshift[k], kSumThreads);
+        }
+        __syncthreads();
+        for (int g = 0; g < nb; ++g) {
+            const size_t row = (size_t)(b0 + g) * N;
+            i64 s[NCH], co[NCH];
+            double acc[NCH];
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                sincos_fix((u64)i0 * det[g][c].step, &s[c], &co[c]);
+                acc[c] = 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < kBins; ++q) {
                 const int i = i0 + q * kSumThreads;
-                if (q > 0) {
-                    const double cn = co * cd - s * sd;
-                    s = fma(s, cd, co * sd);
-                    co = cn;
-                }
                 if (i < N) {
-                    const double2 p = hp[(size_t)b * N + i], c = hc[(size_t)b * N + i];
-                    const double2 d = data[(size_t)ch * N + i];
-                    // (F+ h+ + Fx hx) (co - i s)
-                    const double gr = fp * p.x + fc * c.x, gi = fp * p.y + fc * c.y;
-                    const double rr = d.x - (gr * co + gi * s);
-                    const double ri = d.y - (gi * co - gr * s);
-                    // reciprocal (seed + one Newton step, 3 FP64 instructions)
-                    // and a product instead of a division (about 6)
-                    acc = fma(fma(rr, rr, ri * ri), eob::eob_rcp(psd[(size_t)ch * N + i]), acc);
+                    const double2 p = hp[row + i], x = hc[row + i];
+                    const FdStrain h = fd_strain(p, x);
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) {
+                        const FdDetector &t = det[g][c];
+                        if (q > 0) rotate(&s[c], &co[c], t.rs, t.rc);
+                        double power;
+                        if (h.slow || t.slow || d[q][c].slow) {
+                            const size_t k = (size_t)(first + c) * B + b0 + g;
+                            power = fd_power_slow(p, x, Fplus[k], Fcross[k], data[(size_t)(first + c) * N + i],
+                                                  df * i * tshift[k]);
+                        } else {
+                            power = fd_power(h, t, s[c], co[c], d[q][c]);
+                        }
+                        acc[c] = fma(power, d[q][c].w, acc[c]);
+                    }
                 }
             }
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-            if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = acc;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double t = 0.0;
-                for (int w = 0; w < kSumThreads / 32; ++w) t += warp_sum[w];
-                temp_sum[((size_t)blockIdx.x * B + b) * nch + ch] = make_double2(t, 0.0);
+            for (int c = 0; c < NCH; ++c) {
+                double t = acc[c];
+                for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+                if ((tid & 31) == 0) sums[g][c][tid >> 5] = t;
             }
-            __syncthreads();
+        }
+        __syncthreads();
+        for (int t = tid; t < nb * NCH; t += kSumThreads) {
+            double v = 0.0;
+            for (int k = 0; k < kWarps; ++k) v += sums[t / NCH][t % NCH][k];
+            temp_sum[((size_t)blockIdx.x * B + b0 + t / NCH) * nch + first + t % NCH] = make_double2(v, 0.0);
         }
     }
 }
@@ -248,10 +281,31 @@ int eob_all_in_one_likelihood(double *temp_sum, const double *hp_fd, const doubl
     if (num_bin_all == 0 || nchannels == 0 || data_length == 0) return EOB_OK;
     if (!temp_sum || !hp_fd || !hc_fd || !data || !psd || !Fplus || !Fcross || !time_shift) return EOB_E_ARG;
     const int nblocks = (data_length + kSumBins - 1) / kSumBins;
-    dim3 grid(nblocks, num_bin_all < 65535 ? num_bin_all : 65535, nchannels < 65535 ? nchannels : 65535);
-    k_fd_lnl<<<grid, kSumThreads, 0, stream>>>((double2 *)temp_sum, (const double2 *)hp_fd, (const double2 *)hc_fd,
-                                               (const double2 *)data, psd, Fplus, Fcross, time_shift, df, num_bin_all,
-                                               nchannels, data_length);
+    // binaries per block: enough blocks for four per SM, then as many binaries
+    // as share one conversion of the data
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const long long items = (long long)num_bin_all * nblocks * ((nchannels + 1) / 2);
+    long long group = items / (4LL * (nsm > 0 ? nsm : 1));
+    group = group < 1 ? 1 : (group > kSumGroup ? kSumGroup : group);
+    const long long groups = (num_bin_all + group - 1) / group;
+    const int pairs = nchannels / 2;
+    for (int z = 0; z < pairs; z += 65535) {
+        const dim3 grid(nblocks, (unsigned)(groups < 65535 ? groups : 65535), pairs - z < 65535 ? pairs - z : 65535);
+        k_fd_lnl<2><<<grid, kSumThreads, 0, stream>>>((double2 *)temp_sum, (const double2 *)hp_fd,
+                                                      (const double2 *)hc_fd, (const double2 *)data, psd, Fplus, Fcross,
+                                                      time_shift, df, num_bin_all, (int)group, 2 * z, nchannels,
+                                                      data_length);
+        if (cudaGetLastError() != cudaSuccess) return EOB_E_CUDA;
+    }
+    if (nchannels & 1) {
+        const dim3 grid(nblocks, (unsigned)(groups < 65535 ? groups : 65535), 1);
+        k_fd_lnl<1><<<grid, kSumThreads, 0, stream>>>((double2 *)temp_sum, (const double2 *)hp_fd,
+                                                      (const double2 *)hc_fd, (const double2 *)data, psd, Fplus, Fcross,
+                                                      time_shift, df, num_bin_all, (int)group, nchannels - 1, nchannels,
+                                                      data_length);
+    }
     return ret(cudaGetLastError());
 }
 

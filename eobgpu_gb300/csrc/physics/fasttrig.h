@@ -35,6 +35,24 @@ static __device__ __noinline__ double2 eob_sincos_large(double x)
 }
 #endif
 
+#ifdef __CUDACC__
+// Conversions by integer operations (a conversion instruction takes an FP64
+// issue slot): |x| < 2^127 truncated to a float, below 2^-126 to zero; a float
+// (zero as 2^-127) as a double.
+__device__ __forceinline__ float f32_trunc(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned a = hi & 0x7fffffffu;
+    return __uint_as_float(a < (897u << 20) ? 0u : (hi & 0x80000000u) | ((a - (896u << 20)) << 3) | (lo >> 29));
+}
+
+__device__ __forceinline__ double f64_of(float f)
+{
+    const unsigned b = __float_as_uint(f);
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+#endif
+
 EOB_HD void eob_sincos(double x, double *s, double *c)
 {
 #ifdef __CUDA_ARCH__
@@ -52,10 +70,10 @@ EOB_HD void eob_sincos(double x, double *s, double *c)
     const double r = fma(-kd, EOB_TRIG_STEP_LO, fma(-kd, EOB_TRIG_STEP_HI, x));
     const int i = k & 511;
     const double st = __ldg(&kSinQ[i]), ct = __ldg(&kSinQ[512 - i]);
-    const float rf = (float)r, q = rf * rf;
+    const float rf = f32_trunc(r), q = rf * rf;
     const double r2 = r * r;
-    const double sr = r + (double)(rf * q * fmaf(q, 1.0f / 120.0f, -1.0f / 6.0f));
-    const double c1 = fma(-0.5, r2, (double)(q * q * (1.0f / 24.0f)));
+    const double sr = r + f64_of(rf * q * fmaf(q, 1.0f / 120.0f, -1.0f / 6.0f));
+    const double c1 = fma(-0.5, r2, f64_of(q * q * (1.0f / 24.0f)));
     const double sv = fma(ct, sr, fma(st, c1, st)), cv = fma(-st, sr, fma(ct, c1, ct));
     // quadrant of the multiple: a swap and two sign bits
     const bool odd = (k & 512) != 0;
