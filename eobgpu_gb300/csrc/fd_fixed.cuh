@@ -11,7 +11,7 @@
 //  * dot_hi: a sum of two 64-bit products' upper halves from six 32-bit ones (the
 //    products of the low halves, below the last place, left out).
 //  * The delay phase is exact: f tau in units of 2^-64 turn is an integer product;
-//    sine and cosine come from a table in units of 2^-61, and the next bin of a
+//    sine and cosine come from fasttrig.h in units of 2^-61, and the next bin of a
 //    thread by a rotation (2^-58 a step).
 //    A vector's components share an exponent, so a residual of exactly equal
 //    terms is 2^-57 of their size rather than zero.
@@ -24,10 +24,6 @@
 
 namespace eob {
 
-typedef long long i64;
-typedef unsigned long long u64;
-
-__device__ const i64 kSinFix[513] = EOB_SINFIX_INIT;
 constexpr int kFixTop = 1023 + 960;  // largest exponent field of the integer path
 
 // (a b + c d) / 2^64 for |a|, |c| <= 2^61 and |b|, |d| <= 2^61 (one unit low at most)
@@ -63,29 +59,6 @@ __device__ __forceinline__ u64 turn_of(double u)
     const int sh = e - 1023 - 52 + 64;  // u = m 2^(e - 1023 - 52)
     const u64 t = sh >= 0 ? (sh < 64 ? m << sh : 0ull) : (sh > -64 ? m >> -sh : 0ull);
     return b < 0 ? 0ull - t : t;
-}
-
-// sin and cos of 2 pi t / 2^64 in units of 2^-61 (fasttrig.h's method)
-__device__ __forceinline__ void sincos_fix(u64 t, i64 *s, i64 *c)
-{
-    const u64 v = t + (1ull << 52);
-    const unsigned k = (unsigned)(v >> 53);
-    const i64 rem = (i64)(v & ((1ull << 53) - 1)) - (1ll << 52);
-    const i64 r = __mul64hi(rem << 9, 0x6487ed5110b4611all);  // 2 pi 2^60: the remainder, units of 2^-69
-    const u64 z = (u64)__mul64hi(r, r);                       // r^2, units of 2^-74
-    const unsigned zt = (unsigned)(z >> 24);
-    const unsigned z2 = __umulhi(zt, zt);                     // r^4, units of 2^-68
-    // cos r - 1 = -r^2 / 2 + r^4 / 24 and (sin r - r) / r = -r^2 / 6 + r^4 / 120, units of 2^-74
-    const i64 c1 = (i64)(((u64)z2 * 2863311531u) >> 30) - (i64)(z >> 1);
-    const i64 w = (i64)(((u64)z2 * 2290649225u) >> 32) - (i64)__umul64hi(z, 3074457345618258603ull);
-    const i64 sr = r + (__mul64hi(r, w << 8) >> 18);
-    const int i = k & 511;
-    const i64 st = __ldg(&kSinFix[i]), ct = __ldg(&kSinFix[512 - i]);
-    const i64 sv = st + (__mul64hi(ct, sr) >> 5) + (__mul64hi(st, c1) >> 10);
-    const i64 cv = ct - (__mul64hi(st, sr) >> 5) + (__mul64hi(ct, c1) >> 10);
-    const i64 sa = (k & 512) ? cv : sv, ca = (k & 512) ? sv : cv;
-    *s = (k & 1024) ? -sa : sa;
-    *c = ((k + 512) & 1024) ? -ca : ca;
 }
 
 // (c, s) turned by (rc, rs)

@@ -1,44 +1,33 @@
-// Sine and cosine for FP64 issue rate: 11 FP64 instructions.
+// Sine and cosine without FP64 instructions.
 //
-// On GB300 an FP64 instruction costs an SM sub-partition 64 issue cycles, so
-// the device library's sincos is the largest single piece of a waveform
-// sample.  Here the argument is reduced to the nearest multiple of 2 pi / 2048
-// (Cody and Waite with fused products: the first is exact, since the step's
-// last place divides every intermediate value), the sine and cosine of the
-// multiple come from a quarter-wave table of 513 correctly rounded entries
-// (S. Gal's method, as in Tang's log of fastlog.h), and the angle-addition
-// formulas take the remainder |r| <= pi / 2048:
-//   sin r = r + (-r^3 / 6 + r^5 / 120),  cos r - 1 = -r^2 / 2 + r^4 / 24,
-// the bracketed terms (below 6e-10 and 3e-13) in single precision, whose
-// rounding they bring below 1e-16.  Within 2.2e-16 absolute of the exact values
-// for |x| < 2^40 (tests/test_gpu_sincos.py); larger, infinite and NaN
-// arguments take the library's sincos.  Host: the library.
+// On GB300 an FP64 instruction costs an SM sub-partition 64 issue cycles, a
+// conversion to or from a double as much, an integer one 2 and a 32 x 32 + 64 bit
+// product 4, so the device library's sincos is the largest single piece of a
+// waveform sample (38 FP64 instructions; 11 with a table and FP64 sums).
+// Here the phase becomes an integer, units of 2^-64 turn, by one wide product with
+// 2^64 / (2 pi) to 126 bits; sine and cosine of its nearest multiple of 1 / 2048
+// turn come from a quarter-wave table in units of 2^-61 (S. Gal's method, as
+// in Tang's log of fastlog.h), and the angle-addition formulas take the remainder
+// |r| <= pi / 2048 with
+//   sin r = r - r^3 / 6 + r^5 / 120,  cos r - 1 = -r^2 / 2 + r^4 / 24
+// in 64-bit integers: within 2^-59.7, then rounded to a double (half an ulp, and
+// 2^-59.7 absolute, of the exact values for |x| < 2^40, tests/test_gpu_sincos.py).
+// Larger, infinite and NaN arguments take the library's sincos.  Host: the
+// library.
 #pragma once
 #include "fac_coeffs.h"
 #include "trig_table.h"
 
 namespace eob {
 
+typedef long long i64;
+typedef unsigned long long u64;
+
 #ifdef __CUDACC__
-__device__ const double kSinQ[513] = EOB_SINQ_INIT;
+__device__ const i64 kSinFix[513] = EOB_SINFIX_INIT;
 __device__ const double kArgGammaD[7][EOB_ARG_GAMMA_N] = EOB_ARG_GAMMA_INIT;
-#endif
-static constexpr double kArgGammaH[7][EOB_ARG_GAMMA_N] = EOB_ARG_GAMMA_INIT;
 
-#ifdef __CUDACC__
-// the rare arguments, out of line
-static __device__ __noinline__ double2 eob_sincos_large(double x)
-{
-    double2 r;
-    sincos(x, &r.x, &r.y);
-    return r;
-}
-#endif
-
-#ifdef __CUDACC__
-// Conversions by integer operations (a conversion instruction takes an FP64
-// issue slot): |x| < 2^127 truncated to a float, below 2^-126 to zero; a float
-// (zero as 2^-127) as a double.
+// |x| < 2^127 truncated to a float, below 2^-126 to zero, by integer operations
 __device__ __forceinline__ float f32_trunc(double x)
 {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
@@ -46,42 +35,77 @@ __device__ __forceinline__ float f32_trunc(double x)
     return __uint_as_float(a < (897u << 20) ? 0u : (hi & 0x80000000u) | ((a - (896u << 20)) << 3) | (lo >> 29));
 }
 
-__device__ __forceinline__ double f64_of(float f)
+// the rare arguments, out of line
+static __device__ __noinline__ double2 eob_sincos_large(double x)
 {
-    const unsigned b = __float_as_uint(f);
-    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+    double2 r;
+    sincos(x, &r.x, &r.y);
+    return r;
+}
+
+// x / (2 pi) mod 1 in units of 2^-64, |x| < 2^40: the 53-bit mantissa times
+// 2^64 / (2 pi) (62 integer and 64 fraction bits), shifted by the exponent
+__device__ __forceinline__ u64 turns_of(double x)
+{
+    const i64 b = __double_as_longlong(x);
+    const int e = (int)((b >> 52) & 0x7ff);
+    const u64 m = ((u64)b & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
+    const u64 low = m * 0x28be60db9391054aull, lo = low + __umul64hi(m, 0x7f09d5f47d4d3770ull);
+    const u64 hi = __umul64hi(m, 0x28be60db9391054aull) + (lo < low ? 1 : 0);
+    const int s = 1075 - e;  // 12 .. 1075
+    u64 u = s < 64 ? (lo >> s) | (hi << (64 - s)) : (s < 128 ? hi >> (s - 64) : 0ull);
+    return b < 0 ? 0ull - u : u;
+}
+
+// sin and cos of 2 pi t / 2^64 in units of 2^-61
+__device__ __forceinline__ void sincos_fix(u64 t, i64 *s, i64 *c)
+{
+    const u64 v = t + (1ull << 52);
+    const unsigned k = (unsigned)(v >> 53);
+    const i64 rem = (i64)(v & ((1ull << 53) - 1)) - (1ll << 52);
+    const i64 r = __mul64hi(rem << 9, 0x6487ed5110b4611all);  // 2 pi 2^60: the remainder, units of 2^-69
+    const u64 z = (u64)__mul64hi(r, r);                       // r^2, units of 2^-74
+    const unsigned zt = (unsigned)(z >> 24);
+    const unsigned z2 = __umulhi(zt, zt);                     // r^4, units of 2^-68
+    // cos r - 1 = -r^2 / 2 + r^4 / 24 and (sin r - r) / r = -r^2 / 6 + r^4 / 120, units of 2^-74
+    const i64 c1 = (i64)(((u64)z2 * 2863311531u) >> 30) - (i64)(z >> 1);
+    const i64 w = (i64)(((u64)z2 * 2290649225u) >> 32) - (i64)__umul64hi(z, 3074457345618258603ull);
+    const i64 sr = r + (__mul64hi(r, w << 8) >> 18);
+    const int i = k & 511;
+    const i64 st = __ldg(&kSinFix[i]), ct = __ldg(&kSinFix[512 - i]);
+    const i64 sv = st + (__mul64hi(ct, sr) >> 5) + (__mul64hi(st, c1) >> 10);
+    const i64 cv = ct - (__mul64hi(st, sr) >> 5) + (__mul64hi(ct, c1) >> 10);
+    const i64 sa = (k & 512) ? cv : sv, ca = (k & 512) ? sv : cv;
+    *s = (k & 1024) ? -sa : sa;
+    *c = ((k + 512) & 1024) ? -ca : ca;
+}
+
+// v 2^-61 as a double, |v| < 2^62, rounded to nearest
+__device__ __forceinline__ double unit_value(i64 v)
+{
+    const u64 a = (u64)(v < 0 ? -v : v);
+    const int z = __clzll((i64)a);
+    const u64 m = a << (z & 63);
+    // leading bit 2^(63 - z - 61); it carries into the exponent field, and so does a rounding up
+    const u64 b = ((u64)(unsigned)(1024 - z) << 52) + (m >> 11) + ((m >> 10) & 1);
+    return __longlong_as_double(a == 0 ? 0ll : (i64)(b | ((u64)v & 0x8000000000000000ull)));
 }
 #endif
+static constexpr double kArgGammaH[7][EOB_ARG_GAMMA_N] = EOB_ARG_GAMMA_INIT;
 
 EOB_HD void eob_sincos(double x, double *s, double *c)
 {
 #ifdef __CUDA_ARCH__
-    constexpr double kShift = 6755399441055744.0;  // 1.5 2^52
-    const unsigned xe = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    if (xe >= 0x42700000u) {  // |x| >= 2^40, inf, NaN
+    if ((unsigned)(__double2hiint(x) & 0x7fffffff) >= 0x42700000u) {  // |x| >= 2^40, inf, NaN
         const double2 r = eob_sincos_large(x);
         *s = r.x;
         *c = r.y;
         return;
     }
-    const double t = fma(x, EOB_TRIG_INV, kShift);
-    const double kd = t - kShift;
-    const int k = __double2loint(t);
-    const double r = fma(-kd, EOB_TRIG_STEP_LO, fma(-kd, EOB_TRIG_STEP_HI, x));
-    const int i = k & 511;
-    const double st = __ldg(&kSinQ[i]), ct = __ldg(&kSinQ[512 - i]);
-    const float rf = f32_trunc(r), q = rf * rf;
-    const double r2 = r * r;
-    const double sr = r + f64_of(rf * q * fmaf(q, 1.0f / 120.0f, -1.0f / 6.0f));
-    const double c1 = fma(-0.5, r2, f64_of(q * q * (1.0f / 24.0f)));
-    const double sv = fma(ct, sr, fma(st, c1, st)), cv = fma(-st, sr, fma(ct, c1, ct));
-    // quadrant of the multiple: a swap and two sign bits
-    const bool odd = (k & 512) != 0;
-    const double sa = odd ? cv : sv, ca = odd ? sv : cv;
-    const int sneg = (int)(((unsigned)k << 21) & 0x80000000u);
-    const int cneg = (int)(((unsigned)(k + 512) << 21) & 0x80000000u);
-    *s = __hiloint2double(__double2hiint(sa) ^ sneg, __double2loint(sa));
-    *c = __hiloint2double(__double2hiint(ca) ^ cneg, __double2loint(ca));
+    i64 sf, cf;
+    sincos_fix(turns_of(x), &sf, &cf);
+    *s = unit_value(sf);
+    *c = unit_value(cf);
 #else
     *s = sin(x);
     *c = cos(x);

@@ -1,8 +1,7 @@
 """Write trig_table.h: the tables of eob_sincos and of the Gamma phase.
 
-kSinQ[i] = RN(sin(2 pi i / 2048)), i = 0..512 (a quarter wave; the cosine is
-read backwards), and 2 pi / 2048 as the sum of two doubles.  kSinFix[i] is the same
-value in units of 2^-61.
+kSinFix[i] = sin(2 pi i / 2048) in units of 2^-61, i = 0..512 (a quarter wave;
+the cosine is read backwards).
 
 kArgGamma[l - 2][k]: coefficients, in z = (y / (l + 1))^2, of a polynomial for
 arg Gamma(l + 1 + i y) / y on 0 <= z <= 0.81, l = 2..8.  The function is
@@ -68,11 +67,6 @@ def main():
     print("// Written by gen_trig_table.py: quarter-wave sine table and Gamma-phase polynomials.")
     print("#pragma once")
     step = 2 * mp.pi / 2048
-    hi = mp.mpf(float(step))
-    print(f"#define EOB_TRIG_STEP_HI {float(hi).hex()}")
-    print(f"#define EOB_TRIG_STEP_LO {float(step - hi).hex()}")
-    print(f"#define EOB_TRIG_INV {float(1 / step).hex()}")
-    print("#define EOB_SINQ_INIT { \\\n    " + row([mp.sin(step * i) for i in range(513)]).replace("\n", " \\\n") + "}")
     print("#define EOB_SINFIX_INIT { \\\n    "
           + row([hex(int(mp.nint(mp.sin(step * i) * 2 ** 61))) + "ll" for i in range(513)]).replace("\n", " \\\n") + "}")
     rows = ["{" + row(coefficients(l)).replace("\n", " \\\n") + "}" for l in range(2, 9)]
