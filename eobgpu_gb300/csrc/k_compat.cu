@@ -6,6 +6,7 @@
 //
 // The "SEOBNRv5 class" (src/EOB.cu:3343-3496) is a caller-owned device
 // buffer holding one FacCoeffs table per system (eob_ctx_bytes).
+#include <cooperative_groups.h>
 #include "eob_device.cuh"
 #include "spline_block.cuh"
 #include "physics/hyperdual.h"
@@ -170,7 +171,173 @@ __device__ void rhs_ref(const FacCoeffs *ctx, const double *add, int n, int i, i
     eob_rhs(h, v, y, k);
 }
 
-__global__ void k_ctx_ode(const FacCoeffs *ctx, const double *arg, double *k, const double *add, int n, const int *idx)
+// The right-hand side of 32 systems (lane = system), its work split over the
+// eight one-warp blocks of a cluster: each builds the Hamiltonian
+// coefficients of one group of terms (the compiler drops what a group does not
+// need), block 0 evaluates the Hamiltonian, blocks 0 .. 2 the flux's shared
+// factors, and block m - 1 the multipoles of one m; they meet in block 0's shared
+// memory.  One thread per system ran all of it as one chain of 2838 FP64
+// instructions (64 cycles each) on as few as four SMs.  A warp of a cluster has
+// its SM sub-partition's FP64 pipe to itself; eight warps of one block share four.
+// 512 systems: 109 us -> 47 us in one block -> 35 us in a cluster.
+constexpr int kOdeWarps = 8, kHamDoubles = (int)(sizeof(HamCoeffs) / sizeof(double));
+
+struct OdeShared {
+    double ham[kHamDoubles][32];
+    double dHdr[32], dHdpr[32], omega[32], omega_c[32], Hreal[32];
+    double v[32], lv[32], vp2[10][32], E1[32], sum[kOdeWarps][32];
+};
+
+// the fields of one group of terms, from a full (mostly unused) build
+template <int PART>
+__device__ __forceinline__ void ode_ham_part(OdeShared &sh, const double *add, int n, int i, int lane)
+{
+    HamCoeffs h;
+    ham_of_add(&h, add, n, i);
+    auto put = [&](const double &f) {
+        sh.ham[(int)(&f - reinterpret_cast<const double *>(&h))][lane] = f;
+    };
+    const HamCoeffs::Derived &d = h.d;
+    if constexpr (PART == 0) {
+        put(h.M); put(h.nu); put(h.ak0h); put(d.ak0l6); put(d.ak0l5); put(d.ak0h); put(d.two_nu);
+#pragma unroll
+        for (int k = 0; k < 7; ++k) { put(h.ak0[k]); put(h.ak0l[k]); }
+    } else if constexpr (PART == 1) {
+#pragma unroll
+        for (int k = 0; k < 7; ++k) put(h.aka[k]);
+        put(h.fa1); put(h.fa2); put(h.ap2); put(h.apsq); put(h.kb); put(d.fa2); put(d.two_ap2);
+    } else if constexpr (PART == 2) {
+        put(h.as4); put(h.as5); put(h.as6); put(d.as6); put(d.as5); put(d.as4);
+        put(h.bs3); put(h.bs4); put(d.bs4); put(d.bs3); put(h.dbh); put(d.dbl5); put(d.dbl4); put(d.dbh);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) { put(h.db[k]); put(h.dbl[k]); }
+    } else if constexpr (PART == 3) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) put(h.q4c[k]);
+        put(h.q4l); put(h.q4h); put(d.q4c4); put(d.q4c3); put(d.q4c2); put(d.q4h);
+    } else if constexpr (PART == 4) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) put(h.q6c[k]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) put(h.q8c[k]);
+        put(h.q6h); put(h.q8h); put(d.q6h); put(d.q6c3); put(d.q6c2); put(d.q8h); put(d.q8c2);
+    } else if constexpr (PART == 5) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) { put(h.nc[0][k]); put(h.ncl[0][k]); }
+        put(d.nc02); put(d.nc03); put(d.nc04);
+    } else if constexpr (PART == 6) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) { put(h.nc[1][k]); put(h.ncl[1][k]); put(h.nc[2][k]); put(h.ncl[2][k]); }
+        put(d.nc12); put(d.nc13);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) { put(h.nc[3][k]); put(h.ncl[3][k]); put(h.nc[4][k]); put(h.ncl[4][k]); }
+        put(d.four_n4);
+    }
+}
+
+__global__ void __cluster_dims__(kOdeWarps, 1, 1) __launch_bounds__(32) k_ctx_ode(const FacCoeffs *ctx,
+                                                                                 const double *arg, double *k,
+                                                                                 const double *add, int n,
+                                                                                 const int *idx)
+{
+    __shared__ OdeShared own;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    OdeShared &sh = *cluster.map_shared_rank(&own, 0);
+    const int lane = threadIdx.x, w = (int)cluster.block_rank(), first = (int)(blockIdx.x / kOdeWarps) * 32;
+    const int i = min(first + lane, n - 1);
+    cluster.sync();  // block 0 has started: its shared memory may be written
+    switch (w) {
+        case 0: ode_ham_part<0>(sh, add, n, i, lane); break;
+        case 1: ode_ham_part<1>(sh, add, n, i, lane); break;
+        case 2: ode_ham_part<2>(sh, add, n, i, lane); break;
+        case 3: ode_ham_part<3>(sh, add, n, i, lane); break;
+        case 4: ode_ham_part<4>(sh, add, n, i, lane); break;
+        case 5: ode_ham_part<5>(sh, add, n, i, lane); break;
+        case 6: ode_ham_part<6>(sh, add, n, i, lane); break;
+        default: ode_ham_part<7>(sh, add, n, i, lane); break;
+    }
+    const double r = arg[i], pr = arg[2 * (size_t)n + i], L = arg[3 * (size_t)n + i];
+    cluster.sync();
+    if (w == 0) {
+        HamCoeffs h;
+        double *f = reinterpret_cast<double *>(&h);
+#pragma unroll
+        for (int q = 0; q < kHamDoubles; ++q) f[q] = sh.ham[q][lane];
+        HamEval e;
+        ham_eval(h, r, pr, L, &e);
+        sh.dHdr[lane] = e.dHdr;
+        sh.dHdpr[lane] = e.dHdpr;
+        sh.omega[lane] = e.dHdL;
+        sh.omega_c[lane] = e.omega_c;
+        sh.Hreal[lane] = e.Hreal;
+    }
+    cluster.sync();
+    const double omega = sh.omega[lane], Hreal = sh.Hreal[lane];
+    if (w == 0) {
+        const double ro = eob_rcbrt(omega), v = omega * (ro * ro);
+        sh.v[lane] = v;
+        sh.lv[lane] = eob_log(v);
+    } else if (w == 1) {
+        const double rc = eob_rcbrt(sh.omega_c[lane]), vphi = omega * (rc * rc), p = vphi * vphi;
+        double q = 1.0;
+        sh.vp2[0][lane] = 1.0;
+#pragma unroll
+        for (int j = 1; j < 10; ++j) sh.vp2[j][lane] = q *= p;
+    } else if (w == 2) {
+        sh.E1[lane] = exp(-4.0 * kPi * Hreal * omega);
+    }
+    cluster.sync();
+    const FacFluxView t = flux_view(&ctx[idx ? idx[i] : i], add, n, i, sh.ham[1][lane]);
+    {
+        FluxShared s;
+        s.omega = omega;
+        s.v = sh.v[lane];
+        s.lv = sh.lv[lane];
+        s.Se = fma(Hreal * Hreal - 1.0, t.c_inv2eta(), 1.0);
+        s.Sodd = s.v * L;
+        const double v2 = s.v * s.v, v4 = v2 * v2;
+        s.v12 = v4 * v4 * v4;
+        s.S2e = s.Se * s.Se;
+        s.S2o = s.Sodd * s.Sodd;
+        s.x = 4.0 * kPi * Hreal * omega;
+        double vp2[10];
+#pragma unroll
+        for (int q = 0; q < 10; ++q) vp2[q] = sh.vp2[q][lane];
+        const double hw = Hreal * omega, E1 = sh.E1[lane], E2 = E1 * E1, E4 = E2 * E2;
+        double f;
+        switch (w) {
+            case 0: f = flux_m<1>(t, s, E1, hw, vp2); break;
+            case 1: f = flux_m<2>(t, s, E2, hw, vp2); break;
+            case 2: f = flux_m<3>(t, s, E2 * E1, hw, vp2); break;
+            case 3: f = flux_m<4>(t, s, E4, hw, vp2); break;
+            case 4: f = flux_m<5>(t, s, E4 * E1, hw, vp2); break;
+            case 5: f = flux_m<6>(t, s, E4 * E2, hw, vp2); break;
+            case 6: f = flux_m<7>(t, s, E4 * (E2 * E1), hw, vp2); break;
+            default: f = flux_m<8>(t, s, E4 * E4, hw, vp2); break;
+        }
+        sh.sum[w][lane] = f;
+    }
+    cluster.sync();  // the last remote access
+    if (w != 0 || first + lane >= n) return;
+    double sum = sh.sum[0][lane];
+#pragma unroll
+    for (int q = 1; q < kOdeWarps; ++q) sum += sh.sum[q][lane];
+    const double fo = flux_over_omega(t, sum, omega);
+    k[i] = sh.dHdpr[lane];
+    k[(size_t)n + i] = omega;
+    k[2 * (size_t)n + i] = -fma(pr * eob_rcp(L), fo, sh.dHdr[lane]);
+    k[3 * (size_t)n + i] = -fo;
+}
+
+// The same with one thread per system, for batches that fill the device:
+// a cluster's eight warps repeat what the groups share, so beyond about 32 systems per
+// SM the one chain per thread is the faster (4096 systems: 71 us in clusters, 110 us
+// here; 8192: 111 and 110 us; 16384: 228 and 123 us).
+constexpr int kOdeSystemsPerSm = 32;
+
+__global__ void k_ctx_ode_wide(const FacCoeffs *ctx, const double *arg, double *k, const double *add, int n,
+                               const int *idx)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -580,7 +747,13 @@ int eob_ctx_ode(const void *ctx, const double *x, const double *arg, double *k, 
     (void)x;
     if (!ctx || numSys < 0 || (numSys > 0 && (!arg || !k || !add))) return EOB_E_ARG;
     if (numSys == 0) return EOB_OK;
-    k_ctx_ode<<<nblk(numSys), kTPB, 0, stream>>>((const FacCoeffs *)ctx, arg, k, add, numSys, idx);
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (numSys <= kOdeSystemsPerSm * nsm)
+        k_ctx_ode<<<(numSys + 31) / 32 * kOdeWarps, 32, 0, stream>>>((const FacCoeffs *)ctx, arg, k, add, numSys, idx);
+    else
+        k_ctx_ode_wide<<<nblk(numSys), kTPB, 0, stream>>>((const FacCoeffs *)ctx, arg, k, add, numSys, idx);
     return ret(cudaGetLastError());
 }
 

@@ -289,7 +289,7 @@ __device__ __forceinline__ void spline_sample(const Ws &w, const SynthArgs &sa, 
 }
 
 // lnL: a run of chunks per block, one partial per chunk
-__global__ void __launch_bounds__(kSynthThreads) k_synth_lnl(Ws w, SynthArgs sa)
+__global__ void __launch_bounds__(kSynthThreads, 4) k_synth_lnl(Ws w, SynthArgs sa)
 {
     __shared__ double s_red[kSynthThreads];
     __shared__ int s_range[2];
@@ -560,7 +560,8 @@ cudaError_t launch_synth(const Ws &w, const RunArgs &a, int mode, double *out, c
     void (*kern)(Ws, SynthArgs) = mode == 0 ? (mixed ? k_synth_mixed_lnl : k_synth_lnl)
                                 : mode == 2 ? k_synth_strain<2>
                                             : (mixed ? k_synth_mixed_strain : k_synth_strain<1>);
-    kern<<<nsm * 8, kSynthThreads, 0, s>>>(w, sa);
+    const int blocks = mode == 0 ? resident_blocks(kern, kSynthThreads) : nsm * 8;
+    kern<<<blocks, kSynthThreads, 0, s>>>(w, sa);
     k_finalize<<<(a.B + 3) / 4, 128, 0, s>>>(w, a.B, ndata, mode == 0 ? a.lnl : nullptr, a.status_out);
     return cudaGetLastError();
 }

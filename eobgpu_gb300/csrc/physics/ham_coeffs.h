@@ -70,6 +70,7 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
     const double s11 = c1 * c1 * X1 * X1, s22 = c2 * c2 * X2 * X2, s12 = c1 * c2 * nu;
     const double ap2 = s11 + 2.0 * s12 + s22;
     const double Kn = K * nu;
+    const double K2 = K * K, K4 = K2 * K2, K5 = K4 * K;
     h->M = M;
     h->nu = nu;
     h->ap2 = ap2;
@@ -81,9 +82,9 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
     h->ak0[1] = -2.0 * Kn;
     h->ak0[2] = 4.0 * Kn * (Kn - 1.0);
     h->ak0[3] = 2.0 * nu * (-4.0 * K * K * K * n2 + 8.0 * K * K * nu - 4.0 * K + 1.0);
-    h->ak0[4] = nu * (16.0 * pow(K, 4) * n3 - 48.0 * K * K * K * n2 + 48.0 * K * K * nu - 4.0 * K * (nu + 4.0) -
+    h->ak0[4] = nu * (16.0 * K4 * n3 - 48.0 * K * K * K * n2 + 48.0 * K * K * nu - 4.0 * K * (nu + 4.0) -
                       41.0 * pi2 / 32.0 + 106.0 / 3.0);
-    h->ak0[5] = -32.0 * pow(K, 5) * n5 + 128.0 * pow(K, 4) * n4 + K * K * n3 * (8.0 - 192.0 * K) +
+    h->ak0[5] = -32.0 * K5 * n5 + 128.0 * K4 * n4 + K * K * n3 * (8.0 - 192.0 * K) +
                 n2 * (12288.0 * K * K - 7552.0 * K + 246.0 * pi2 * K - 3536.0 + 123.0 * pi2) / 96.0 +
                 nu * (-32.0 * K + 1.0 / 20.0 + 128.0 * eg / 5.0 + 963.0 * pi2 / 512.0 + 256.0 * l2 / 5.0);
     h->ak0l[5] = -64.0 * nu / 5.0;
@@ -99,7 +100,7 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
                 2.0 * nu * km1 * km1 * ap2 * (16.0 * K * K * K * n2 - 36.0 * K * K * nu + 20.0 * K - 1.0);
     h->aka[6] = -Kn * (Kn - 2.0) * km1 * km1 * km1 * km1 * ap2 * ap2 * ap2 -
                 nu * km1 * km1 * ap2 *
-                    (7680.0 * pow(K, 4) * n3 - 24576.0 * K * K * K * n2 + 26112.0 * K * K * nu - 768.0 * K * (nu + 12.0) -
+                    (7680.0 * K4 * n3 - 24576.0 * K * K * K * n2 + 26112.0 * K * K * nu - 768.0 * K * (nu + 12.0) -
                      123.0 * pi2 + 3776.0) / 96.0;
 
     // ---- A factors (src/EOB.cu:92)
