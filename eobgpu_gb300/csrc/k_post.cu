@@ -85,9 +85,9 @@ struct ModeArgs {
 // evaluations in one kernel cost the others their registers and half the
 // instruction cache (five modes, 4096 binaries, splines included: 5.8 ms
 // against 4.2 ms).  FP64 issue bounds both: five modes and the Hamiltonian
-// take 645 FP64 instructions a row in the closed form, 2427 by the sums on
-// every row (4096 binaries: 9.32 ms -> 2.49 + 0.56 ms; 1024 ragged binaries,
-// (2,2) alone: 0.77 -> 0.36 + 0.07 ms).
+// take 585 FP64 instructions a row in the closed form, 2427 by the sums on
+// every row (4096 binaries: 9.32 ms -> 2.25 + 0.47 ms; 1024 ragged binaries,
+// (2,2) alone: 0.77 -> 0.33 + 0.07 ms).
 __global__ void __launch_bounds__(128) k_modes(Ws w, int B, ModeArgs ma)
 {
     const long long R = (long long)w.queue[1];
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(128) k_modes_close(Ws w, int B, ModeArgs ma)
             const int l = ma.ells[j], m = ma.mms[j];
             const int li = lm_index(l, m);
             const cdbl hl = mode_eval_sums(w.fac[b], l, m, rec.pre_re[li], rec.pre_im[li], rec.nu, phi, pphi, v, vh,
-                                           e.Hreal, vPhi, lfact[l], 0.0, true);
+                                           e.Hreal, vPhi, ma.mc[j].y0, lfact[l], 0.0, true);
             w.ys[(size_t)(1 + 2 * j) * Rc + r] = hl.re;
             w.ys[(size_t)(2 + 2 * j) * Rc + r] = hl.im;
         }

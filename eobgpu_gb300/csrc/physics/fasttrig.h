@@ -26,6 +26,7 @@ typedef unsigned long long u64;
 #ifdef __CUDACC__
 __device__ const i64 kSinFix[513] = EOB_SINFIX_INIT;
 __device__ const double kArgGammaD[7][EOB_ARG_GAMMA_N] = EOB_ARG_GAMMA_INIT;
+__device__ const double kArgGammaLowD[7][EOB_ARG_GAMMA_LOW_N] = EOB_ARG_GAMMA_LOW_INIT;
 
 // |x| < 2^127 truncated to a float, below 2^-126 to zero, by integer operations
 __device__ __forceinline__ float f32_trunc(double x)
@@ -92,6 +93,7 @@ __device__ __forceinline__ double unit_value(i64 v)
 }
 #endif
 static constexpr double kArgGammaH[7][EOB_ARG_GAMMA_N] = EOB_ARG_GAMMA_INIT;
+static constexpr double kArgGammaLowH[7][EOB_ARG_GAMMA_LOW_N] = EOB_ARG_GAMMA_LOW_INIT;
 
 EOB_HD void eob_sincos(double x, double *s, double *c)
 {
@@ -123,6 +125,20 @@ EOB_HD double arg_gamma_over_y(int l, double z)
     double p = a[EOB_ARG_GAMMA_N - 1];
 #pragma unroll
     for (int k = EOB_ARG_GAMMA_N - 2; k >= 0; --k) p = fma(p, z, a[k]);
+    return p;
+}
+
+// the same for z <= EOB_ARG_GAMMA_ZLOW
+EOB_HD double arg_gamma_over_y_low(int l, double z)
+{
+#ifdef __CUDA_ARCH__
+    const double *a = kArgGammaLowD[l - 2];
+#else
+    const double *a = kArgGammaLowH[l - 2];
+#endif
+    double p = a[EOB_ARG_GAMMA_LOW_N - 1];
+#pragma unroll
+    for (int k = EOB_ARG_GAMMA_LOW_N - 2; k >= 0; --k) p = fma(p, z, a[k]);
     return p;
 }
 

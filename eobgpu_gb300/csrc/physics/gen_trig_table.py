@@ -7,7 +7,8 @@ kArgGamma[l - 2][k]: coefficients, in z = (y / (l + 1))^2, of a polynomial for
 arg Gamma(l + 1 + i y) / y on 0 <= z <= 0.81, l = 2..8.  The function is
 analytic there (nearest singularity z = -1, the pole of Gamma at 0), so the
 Chebyshev interpolant of degree 19 is within 3e-17 of it, relative to its
-value; it is converted to powers of z at 60 digits.
+value; it is converted to powers of z at 60 digits.  kArgGammaLow: the same on
+0 <= z <= 0.125, where most of an inspiral lies, of degree 10.
 
 Values come from mpmath; the output is hexadecimal floating point, so the
 header is the same on every machine.
@@ -18,6 +19,7 @@ import mpmath as mp
 
 mp.mp.dps = 60
 DEG, ZMAX = 19, mp.mpf("0.81")
+DEG_LOW, ZLOW = 10, mp.mpf("0.125")
 
 
 def arg_gamma_over_y(l, z):
@@ -54,8 +56,8 @@ def fit(f, n, zmax, tol):
     return pz
 
 
-def coefficients(l):
-    return fit(lambda z: arg_gamma_over_y(l, z), DEG + 1, ZMAX, mp.mpf("3e-17"))
+def coefficients(l, deg, zmax):
+    return fit(lambda z: arg_gamma_over_y(l, z), deg + 1, zmax, mp.mpf("3e-17"))
 
 
 def row(v, per=4):
@@ -69,10 +71,11 @@ def main():
     step = 2 * mp.pi / 2048
     print("#define EOB_SINFIX_INIT { \\\n    "
           + row([hex(int(mp.nint(mp.sin(step * i) * 2 ** 61))) + "ll" for i in range(513)]).replace("\n", " \\\n") + "}")
-    rows = ["{" + row(coefficients(l)).replace("\n", " \\\n") + "}" for l in range(2, 9)]
-    print(f"#define EOB_ARG_GAMMA_N {DEG + 1}")
-    print(f"#define EOB_ARG_GAMMA_ZMAX {float(ZMAX)!r}")
-    print("#define EOB_ARG_GAMMA_INIT { \\\n    " + ", \\\n    ".join(rows) + "}")
+    for tag, deg, zmax in (("", DEG, ZMAX), ("_LOW", DEG_LOW, ZLOW)):
+        rows = ["{" + row(coefficients(l, deg, zmax)).replace("\n", " \\\n") + "}" for l in range(2, 9)]
+        print(f"#define EOB_ARG_GAMMA{tag}_N {deg + 1}")
+        print(f"#define EOB_ARG_GAMMA_Z{tag[1:] or 'MAX'} {float(zmax)!r}")
+        print(f"#define EOB_ARG_GAMMA{tag}_INIT {{ \\\n    " + ", \\\n    ".join(rows) + "}")
 
 
 main()

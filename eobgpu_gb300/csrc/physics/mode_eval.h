@@ -80,9 +80,11 @@ EOB_HD void cloggamma_shifted(double zr, double zi, double *lg_re, double *lg_im
 }
 
 // h_lm (or h_lm e^{i m phi} when derotate) with T_lm from the sums of log Gamma, exp() and the
-// library's logarithms.  vh = (H_real v^3)^(1/3), lfact = log(l!), i = lm_index(l, m)
+// library's logarithms.  vh = (H_real v^3)^(1/3), y0 = (-1)^m Y_{l-eps}^m(pi/2, 0),
+// lfact = log(l!), i = lm_index(l, m)
 EOB_HD cdbl mode_eval_sums(const FacCoeffs &fc, int l, int m, double pre_re, double pre_im, double eta, double phi,
-                           double pphi, double v, double vh, double Hreal, double vPhi, double lfact, double h22_calib,
+                           double pphi, double v, double vh, double Hreal, double vPhi, double y0, double lfact,
+                           double h22_calib,
                            bool derotate)
 {
     if (eta > 0.25 && eta < 0.25 + 1e-4) eta = 0.25;
@@ -95,16 +97,22 @@ EOB_HD cdbl mode_eval_sums(const FacCoeffs &fc, int l, int m, double pre_re, dou
     // |Y| part and Newtonian amplitude: n_lm vPhi^(l+eps) (-1)^m Y_{l-eps}^m(pi/2, 0)
     double vpow = 1.0;
     for (int q = 0; q < l + eps; ++q) vpow *= vPhi;
-    const double y0 = ((m % 2) ? -1.0 : 1.0) * ylm_equator(l - eps, m);
     const double S = (eps == 0) ? (Hreal * Hreal - 1.0) / (2.0 * eta) + 1.0 : v * pphi;
     // delta_lm
-    double delta = 0.0, p = 1.0;
-    for (int k = 1; k < 10; ++k) { p *= vh; delta = fma(fc.dvh[i][k], p, delta); }
-    p = 1.0;
-    for (int k = 1; k < 9; ++k) { p *= v; delta = fma(fc.dv[i][k], p, delta); }
+    // (the builder assigns vh^3, vh^6, vh^9 and v^5 only; the powers by one product each, as ever)
+    double p = vh * vh * vh;
+    double delta = fc.dvh[i][3] * p;
+    p = p * vh * vh * vh;
+    delta = fma(fc.dvh[i][6], p, delta);
+    p = p * vh * vh * vh;
+    delta = fma(fc.dvh[i][9], p, delta);
+    p = v * v * v * v * v;
+    delta = fma(fc.dv[i][5], p, delta);
     // rho_lm^l + f_lm
     double rho = 0.0;
-    for (int k = kRhoDeg; k >= 1; --k) rho = (rho + fma(fc.rhol[i][k], eulerlog, fc.rho[i][k])) * v;
+#pragma unroll
+    for (int k = 10; k >= 1; --k)
+        rho = (rho + ((k == 6 || k == 8 || k == 10) ? fma(fc.rhol[i][k], eulerlog, fc.rho[i][k]) : fc.rho[i][k])) * v;
     rho += 1.0;
     if (l == 2 && m == 2) {
         const double v4 = v2 * v2;
@@ -113,8 +121,16 @@ EOB_HD cdbl mode_eval_sums(const FacCoeffs &fc, int l, int m, double pre_re, dou
     double rpl = rho;
     for (int q = 1; q < l; ++q) rpl *= rho;
     double fr = 0.0;
-    p = 1.0;
-    for (int k = 1; k < 8; ++k) { p *= v; fr = fma(fc.fre[i][k], p, fr); }
+    if (l <= 5) {  // f from v^1 and v^3 .. v^6
+        fr = fc.fre[i][1] * v;
+        p = v * v * v;
+        fr = fma(fc.fre[i][3], p, fr);
+#pragma unroll
+        for (int k = 4; k <= 6; ++k) {
+            p *= v;
+            fr = fma(fc.fre[i][k], p, fr);
+        }
+    }
     const double fi = fc.fim_vh6[i] * vh3 * vh3;
     cdbl rf = {rpl + fr, fi};
     if (eta == 0.25 && (m % 2)) rf = {fr, fi};
@@ -161,6 +177,7 @@ struct ModeConst {
     double elog;   // gamma + log(2 m)
     double tail;   // log(4 m / sqrt(e))
     double y0;     // (-1)^m Y_{l-eps}^m(pi/2, 0)
+    double m, il;  // m, 1 / (l + 1)
     double ifact;  // 1 / l!
 };
 
@@ -170,6 +187,8 @@ EOB_HD ModeConst mode_const(int l, int m)
     c.elog = kEulerGamma + log(2.0 * m);
     c.tail = log(4.0 * m / 1.6487212707001281468);  // sqrt(e)
     c.y0 = ((m % 2) ? -1.0 : 1.0) * ylm_equator(l - (l + m) % 2, m);
+    c.m = (double)m;
+    c.il = 1.0 / (l + 1);
     c.ifact = 1.0;
     for (int q = 2; q <= l; ++q) c.ifact /= (double)q;
     return c;
@@ -188,14 +207,21 @@ EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, co
     delta = fma(fc.dv[i][5], v2 * v2 * v, delta);
     // rho_lm^l + f_lm (rho up to v^10, eulerlog parts at v^6, v^8, v^10; f from v^1 and v^3..v^6, l <= 5)
     const double el = mc.elog + w.lv;
-    double rho = fma(fc.rhol[i][10], el, fc.rho[i][10]);
-#pragma unroll
-    for (int k = 9; k >= 1; --k) {
-        double ck = fc.rho[i][k];
-        if (k == 6 || k == 8) ck = fma(fc.rhol[i][k], el, ck);
-        rho = fma(rho, v, ck);
+    const double c10 = fma(fc.rhol[i][10], el, fc.rho[i][10]), c8 = fma(fc.rhol[i][8], el, fc.rho[i][8]),
+                 c6 = fma(fc.rhol[i][6], el, fc.rho[i][6]);
+    double rho;
+    if ((l == m && (l & 1) == 0) || (l == 3 && m == 2) || (l == 4 && m == 2)) {
+        // odd powers too
+        const double *c = fc.rho[i];
+        rho = fma(fma(c10, v, c[9]), v, c8);
+        rho = fma(fma(rho, v, c[7]), v, c6);
+        rho = fma(fma(rho, v, c[5]), v, c[4]);
+        rho = fma(fma(rho, v, c[3]), v, c[2]);
+        rho = fma(rho, v, c[1]) * v;
+    } else {
+        rho = fma(fma(fma(fma(c10, v2, c8), v2, c6), v2, fc.rho[i][4]), v2, fc.rho[i][2]) * v2;
     }
-    rho = fma(rho, v, 1.0);
+    rho += 1.0;
     if (l == 2 && m == 2) {
         const double v4 = v2 * v2;
         rho = fma(h22_calib, v4 * v4 * v4, rho);
@@ -211,14 +237,20 @@ EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, co
     cdbl rf = {rpl + fr, fi};
     if (eta == 0.25 && (m % 2)) rf = {fr, fi};
     // T_lm: its modulus and its phase without the logarithm's term
-    const double k = m * w.Omega, hk = w.Hreal * k, y = 2.0 * hk;
+    const double k = mc.m * w.Omega, hk = w.Hreal * k, y = 2.0 * hk;
     double tmod, targ;
-    const double q = y * (1.0 / (l + 1)), z = q * q;
+    const double q = y * mc.il, z = q * q;
     if (y >= 0.0 && z <= EOB_ARG_GAMMA_ZMAX) {
-        targ = -y * arg_gamma_over_y(l, z);
+        targ = -y * (z <= EOB_ARG_GAMMA_ZLOW ? arg_gamma_over_y_low(l, z) : arg_gamma_over_y(l, z));
         const double y2 = y * y, x = 2.0 * kPi * y;
-        double p = 1.0;
-        for (int j = 1; j <= l; ++j) p *= y2 + (double)(j * j);
+        double p = y2 + 1.0;
+        if (l >= 2) p *= y2 + 4.0;
+        if (l >= 3) p *= y2 + 9.0;
+        if (l >= 4) p *= y2 + 16.0;
+        if (l >= 5) p *= y2 + 25.0;
+        if (l >= 6) p *= y2 + 36.0;
+        if (l >= 7) p *= y2 + 49.0;
+        if (l >= 8) p *= y2 + 64.0;
 #ifdef __CUDA_ARCH__
         const double t2 = x * eob_rcp(-eob_expm1_neg(x)) * p;
         tmod = t2 * eob_rsqrt(t2) * mc.ifact;
@@ -231,7 +263,7 @@ EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, co
         tmod = exp(kPi * hk + lgr) * mc.ifact;
     }
     double phase = fma(y, fma(3.0, w.lv, mc.tail), targ) + delta;
-    if (!derotate) phase -= m * w.phi;
+    if (!derotate) phase -= mc.m * w.phi;
     double sp, cp;
     eob_sincos(phase, &sp, &cp);
     double vpow = 1.0;
