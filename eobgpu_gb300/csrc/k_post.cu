@@ -203,26 +203,33 @@ struct PackedSplines {
     }
 };
 
-constexpr int kSplineThreads = 64, kSplineChunk = 13;
-using PackedBlock = SplineBlock<1, kSplineThreads, kSplineChunk>;
+constexpr int kSplineThreads = 64, kSplineChunk = 9, kSplineShort = kSplineThreads * kSplineChunk;
+constexpr int kSplineLongThreads = 256;
 
 // One block per binary and group of `per` series, in the caller's queue order
-// (longest first: several tiles long, they would end the launch).  64 threads
-// of up to 13 rows: 832 rows a tile, which most trajectories fit (520 rows in
-// 9 per thread); 128 threads of 5 rows would spend a quarter more FP64 issue
-// slots on the scans.  Measured: 4096 binaries, 11 series, 520 rows: 4.67 ms
-// -> 1.09 ms (80 % of the FP64 issue slots); 1024 ragged binaries, 3 series:
-// 0.81 -> 0.39 ms (the longest, 4 tiles, ends it).
-__global__ void __launch_bounds__(kSplineThreads) k_spline(Ws w, const int *order, int nsubs, int nmain, int per,
-                                                           int mixed)
+// (longest first).  NT = 64 threads of up to 9 rows: 576 rows a tile, which most
+// trajectories fit; 128 threads of 5 rows would spend a quarter more FP64 issue
+// slots on the scans, and chunks of 13 rows hold their factors in 250 registers (four
+// blocks on an SM; six with the 168 of a bound of five, which spills 100 bytes).
+// Longer ones go to 256 threads (2304 rows a tile) in a launch of their own: on 64
+// threads the longest of a ragged batch, four tiles one after the other, ended the
+// launch late; 128 threads, or chunks of 5 rows, took 0.03 to 0.06 ms more.
+// 1024 ragged binaries, 3 series: 0.81 ms with a warp per series, 0.39 on 64 threads of
+// 13 rows for all, 0.26 so; 4096 binaries, 11 series, 520 rows: 4.67, 1.19
+// and 1.08 + 0.03 ms (79 % of the FP64 issue slots).
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 64 ? 5 : 1) k_spline(Ws w, const int *order, int nsubs, int nmain, int per, int mixed)
 {
-    __shared__ PackedBlock::Smem sm;
+    using Block = SplineBlock<1, NT, kSplineChunk>;
+    extern __shared__ __align__(16) char smem[];
+    typename Block::Smem &sm = *reinterpret_cast<typename Block::Smem *>(smem);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) w.queue[6] = (unsigned long long)mixed;
     const int b = order ? order[blockIdx.x] : blockIdx.x;
-    const PackedSplines acc{w, w.npts[b] > 0 ? w.nsteps[b] : 0, nmain, (size_t)w.row_off[b],
-                            (size_t)w.L.Bc * (size_t)w.L.Lc, mixed != 0};
+    const int n = w.npts[b] > 0 ? w.nsteps[b] : 0;
+    if ((n > kSplineShort) != (NT > kSplineThreads)) return;
+    const PackedSplines acc{w, n, nmain, (size_t)w.row_off[b], (size_t)w.L.Bc * (size_t)w.L.Lc, mixed != 0};
     const int s0 = blockIdx.y * per;
-    PackedBlock::run(acc, sm, s0, min(nsubs, s0 + per));
+    Block::run(acc, sm, s0, min(nsubs, s0 + per));
 }
 
 cudaError_t launch_prepare_post(const Ws &w, const RunArgs &a, cudaStream_t s)
@@ -247,8 +254,17 @@ cudaError_t launch_prepare_post(const Ws &w, const RunArgs &a, cudaStream_t s)
         const int groups = a.B >= 2 * nsm ? 1 : (2 * nsm + a.B - 1) / a.B;
         per = (nsubs + groups - 1) / groups;
     }
-    k_spline<<<dim3(a.B, (nsubs + per - 1) / per), kSplineThreads, 0, s>>>(w, a.order, nsubs, nmain, per,
-                                                                          a.opt.precision == 1 ? 1 : 0);
+    const int mixed = a.opt.precision == 1 ? 1 : 0;
+    const dim3 grid(a.B, (nsubs + per - 1) / per);
+    using Short = SplineBlock<1, kSplineThreads, kSplineChunk>::Smem;
+    using Long = SplineBlock<1, kSplineLongThreads, kSplineChunk>::Smem;
+    if (w.L.Lc > kSplineShort) {
+        const cudaError_t e = cudaFuncSetAttribute(k_spline<kSplineLongThreads>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Long));
+        if (e != cudaSuccess) return e;
+        k_spline<kSplineLongThreads><<<grid, kSplineLongThreads, sizeof(Long), s>>>(w, a.order, nsubs, nmain, per, mixed);
+    }
+    k_spline<kSplineThreads><<<grid, kSplineThreads, sizeof(Short), s>>>(w, a.order, nsubs, nmain, per, mixed);
     return cudaGetLastError();
 }
 
