@@ -31,7 +31,7 @@ constexpr int kFill = 4096;        // samples past the templates' ends per fill 
 
 struct SynthArgs {
     int B, N, K;
-    int mms[kMaxModes], mmax;
+    int mms[kMaxModes];
     double dt, amp;
     const double *data;   // lnL mode
     double *out;          // strain modes
@@ -211,72 +211,50 @@ struct BinaryGrid {
 };
 
 // The modes of one sample in interval o = base + i at offset xx: per mode
-// (MODE 2) into `put`, else their sum.  FP64 issue bounds it (74 % of the
-// slots): 1024 ragged binaries, (2,2), 11 M samples: 1.43 -> 0.59 ms; 64 binaries,
-// five modes with the merger-ringdown, strain of 24576 samples: 0.50 -> 0.20 ms.
-// For one mode 25 FP64 instructions (the phase 3,
-// sine and cosine 11, two amplitude splines 6, the rotation 2 or 4), 62 with the
-// library's sincos and products for the powers of xx.  Several modes share one
-// sincos: e^{i m phi} for m = 1 .. mmax by complex products (4 FP64
-// instructions each; a mode whose NQC phase enters takes its own sincos).
+// (MODE 2) into `put`, else their sum.  The phase takes 3 FP64 instructions, a mode
+// 8 to 10 (two amplitude splines 6, the rotation 2 or 4; the NQC correction about 30
+// for a sample and 9 for a mode); one mode took 62 with the library's sincos and products
+// for the powers of xx.  Sines and cosines come from the integer phase
+// (fasttrig.h), shared by modes of one m that follow one another.  FP64 issue
+// (66 % of the slots) and the integers (33 % of all issue slots) bound it: 1024 ragged
+// binaries, (2,2), 11 M samples: 1.43 -> 0.28 ms; 64 binaries, five modes with the
+// merger-ringdown, strain of 24576 samples: 0.50 -> 0.14 ms.
 template <int MODE, class Put>
 __device__ __forceinline__ void spline_sample(const Ws &w, const SynthArgs &sa, const ImrRec *recs, size_t Rc, size_t o,
                                               double xx, double *hsum, double *hsum_i, Put put)
 {
     const double phi = cubic(w.ys, w.cA, w.cB, w.cC, o, xx);
     double h = 0.0, hi = 0.0;
-    if (!recs && sa.K > 1) {
-        double s1, c1;
-        eob_sincos(phi, &s1, &c1);
-        double pc = c1, ps = s1;
-        for (int m = 1; m <= sa.mmax; ++m) {
-            if (m > 1) {
-                const double cn = fma(pc, c1, -(ps * s1));
-                ps = fma(ps, c1, pc * s1);
-                pc = cn;
-            }
-            for (int q = 0; q < sa.K; ++q) {
-                if (sa.mms[q] != m) continue;
-                const double re = cubic(w.ys, w.cA, w.cB, w.cC, (size_t)(1 + 2 * q) * Rc + o, xx);
-                const double im = cubic(w.ys, w.cA, w.cB, w.cC, (size_t)(2 + 2 * q) * Rc + o, xx);
-                // (re + i im) e^{-i m phi}
-                if (MODE == 2) put(q, fma(re, pc, im * ps), fma(im, pc, -(re * ps)));
-                else {
-                    h = fma(re, pc, fma(im, ps, h));
-                    if (MODE == 1) hi = fma(im, pc, fma(-re, ps, hi));
-                }
+    const PhaseTurns phase(phi);
+    if (!recs) {
+        double sp = 0.0, cp = 0.0;
+        for (int q = 0; q < sa.K; ++q) {
+            if (q == 0 || sa.mms[q] != sa.mms[q - 1]) phase.multiple(sa.mms[q], &sp, &cp);
+            const double re = cubic(w.ys, w.cA, w.cB, w.cC, (size_t)(1 + 2 * q) * Rc + o, xx);
+            const double im = cubic(w.ys, w.cA, w.cB, w.cC, (size_t)(2 + 2 * q) * Rc + o, xx);
+            // (re + i im) e^{-i m phi}
+            if (MODE == 2) put(q, fma(re, cp, im * sp), fma(im, cp, -(re * sp)));
+            else {
+                h = fma(re, cp, fma(im, sp, h));
+                if (MODE == 1) hi = fma(im, cp, fma(-re, sp, hi));
             }
         }
     } else {
         // NQC correction (EOBNonQCCorrection, eob/seobnrv4phm.py:1686-1700):
         // modulus 1 + (p_r / (r om))^2 (a1 + a2 / r + a3 / r^(3/2)), phase
         // p_r / (r om) (b1 + b2 p_r^2)
-        double p0 = 0.0, p02 = 0.0, pr2 = 0.0, ir = 0.0, ir32 = 0.0;
-        if (recs) {
-            const double om = fma(fma(3.0 * w.cC[o], xx, 2.0 * w.cB[o]), xx, w.cA[o]);
-            const double rr = cubic(w.imr_ys, w.imr_cA, w.imr_cB, w.imr_cC, o, xx);
-            const double pr = cubic(w.imr_ys, w.imr_cA, w.imr_cB, w.imr_cC, Rc + o, xx);
-            const double rs = eob_rsqrt(rr);
-            ir = rs * rs;
-            ir32 = ir * rs;
-            p0 = pr * eob_rcp(rr * om);
-            p02 = p0 * p0;
-            pr2 = pr * pr;
-        }
+        const double om = fma(fma(3.0 * w.cC[o], xx, 2.0 * w.cB[o]), xx, w.cA[o]);
+        const double rr = cubic(w.imr_ys, w.imr_cA, w.imr_cB, w.imr_cC, o, xx);
+        const double pr = cubic(w.imr_ys, w.imr_cA, w.imr_cB, w.imr_cC, Rc + o, xx);
+        const double rs = eob_rsqrt(rr), ir = rs * rs, ir32 = ir * rs;
+        const double p0 = pr * eob_rcp(rr * om), p02 = p0 * p0, pr2 = pr * pr;
         for (int q = 0; q < sa.K; ++q) {
             const double re = cubic(w.ys, w.cA, w.cB, w.cC, (size_t)(1 + 2 * q) * Rc + o, xx);
             const double im = cubic(w.ys, w.cA, w.cB, w.cC, (size_t)(2 + 2 * q) * Rc + o, xx);
-            double ph = sa.mms[q] * phi, sp, cp, mag = 1.0;
-            if (recs) {
-                ph = fma(-p0, fma(recs[q].b2, pr2, recs[q].b1), ph);
-                mag = fma(p02, fma(recs[q].a3, ir32, fma(recs[q].a2, ir, recs[q].a1)), 1.0);
-            }
-            eob_sincos(ph, &sp, &cp);
-            double a = fma(re, cp, im * sp), b = MODE == 0 ? 0.0 : fma(im, cp, -(re * sp));
-            if (recs) {
-                a *= mag;
-                if (MODE != 0) b *= mag;
-            }
+            const double mag = fma(p02, fma(recs[q].a3, ir32, fma(recs[q].a2, ir, recs[q].a1)), 1.0);
+            double sp, cp;
+            phase.multiple(sa.mms[q], -p0 * fma(recs[q].b2, pr2, recs[q].b1), &sp, &cp);
+            const double a = fma(re, cp, im * sp) * mag, b = MODE == 0 ? 0.0 : fma(im, cp, -(re * sp)) * mag;
             if (MODE == 2) put(q, a, b);
             else {
                 h += a;
@@ -412,7 +390,7 @@ __device__ __forceinline__ float turns_to_radians(unsigned long long u)
 // low bits of the sum with 1.5 2^16; multiples of it are integer products,
 // which wrap as the angle does, so every mode's reduction is free (the FP64
 // reduction of each took 5 instructions of the 37 a five-mode sample had; 10 are
-// left: 4096 binaries, five modes, 12 M samples: 0.95 -> 0.40 ms).
+// left: 4096 binaries, five modes, 12 M samples: 0.95 -> 0.36 ms).
 __device__ __forceinline__ void mixed_sample(const Ws &w, const SynthArgs &sa, size_t Rc, size_t o, double xx,
                                              float *h_re, float *h_im)
 {
@@ -549,9 +527,7 @@ cudaError_t launch_synth(const Ws &w, const RunArgs &a, int mode, double *out, c
     sa.B = a.B;
     sa.N = a.N;
     sa.K = a.K;
-    sa.mmax = 0;
     for (int j = 0; j < kMaxModes; ++j) sa.mms[j] = a.mms[j];
-    for (int j = 0; j < a.K; ++j) sa.mmax = a.mms[j] > sa.mmax ? a.mms[j] : sa.mmax;
     sa.dt = a.dt;
     sa.amp = a.amp;
     sa.data = a.data;

@@ -33,61 +33,28 @@ __device__ __forceinline__ double cubic(const double *y, const double *c1, const
 }
 
 // sum_k (re_k + i im_k) e^{-i m_k phi} of one sample; sub-series k of a
-// binary's block start at base + k * stride.  e^{i q phi} for q = 1 .. max m
-// by complex products of e^{i phi} (one sincos of 11 FP64 instructions per
-// sample, fasttrig.h; the powers agree with direct evaluation to ~q ulp), each
-// mode taken at its own q; modes with m outside 1..8 use their own sincos.
-// FP64 issue bounds it: two modes take 42 FP64 instructions a sample, 72 with
-// the library's sincos and products for the powers of x.
+// binary's block start at base + k * stride.  The rotations come from the integer
+// phase (fasttrig.h); a mode with the m of the one before shares its.  FP64 issue
+// bounds it (88 %): two modes take 24 FP64 instructions a sample, 72 with the
+// library's sincos and products for the powers of x, 28 with integer sincos and
+// complex products from one multiple to the next (128 binaries, two modes, 32768
+// samples: 0.36, 0.18 and 0.145 ms).
 __device__ __forceinline__ double2 mode_sum(const double *y, const double *c1, const double *c2, const double *c3,
-                                            size_t base, size_t stride, int ind, double x, int K, const int *ms,
-                                            int mmax)
+                                            size_t base, size_t stride, int ind, double x, int K, const int *ms)
 {
+    // one mode: the phase m phi is rounded once, as a single series' caller would
     const double phi = cubic(y, c1, c2, c3, base + 2 * (size_t)K * stride + ind, x);
-    double hr = 0.0, hi = 0.0;
-    auto add = [&](int k, double c, double s) {
+    const eob::PhaseTurns phase(K == 1 ? ms[0] * phi : phi);
+    double hr = 0.0, hi = 0.0, c = 0.0, s = 0.0;
+    for (int k = 0; k < K; ++k) {
+        if (k == 0 || ms[k] != ms[k - 1]) phase.multiple(K == 1 ? 1 : ms[k], &s, &c);
         const double re = cubic(y, c1, c2, c3, base + (size_t)k * stride + ind, x);
         const double im = cubic(y, c1, c2, c3, base + (size_t)(K + k) * stride + ind, x);
         // (re + i im)(c - i s)
         hr = fma(re, c, fma(im, s, hr));
         hi = fma(im, c, fma(-re, s, hi));
-    };
-    if (K == 1) {
-        double s, c;
-        eob::eob_sincos(ms[0] * phi, &s, &c);
-        add(0, c, s);
-        return make_double2(hr, hi);
-    }
-    if (mmax > 0) {
-        double s1, cp1;
-        eob::eob_sincos(phi, &s1, &cp1);
-        double pc = cp1, ps = s1;
-        for (int q = 1;; ++q) {
-            for (int k = 0; k < K; ++k)
-                if (ms[k] == q) add(k, pc, ps);
-            if (q == mmax) break;
-            const double cn = fma(pc, cp1, -(ps * s1));
-            ps = fma(ps, cp1, pc * s1);
-            pc = cn;
-        }
-    }
-    for (int k = 0; k < K; ++k) {
-        if (ms[k] < 1 || ms[k] > 8) {
-            double s, c;
-            eob::eob_sincos(ms[k] * phi, &s, &c);
-            add(k, c, s);
-        }
     }
     return make_double2(hr, hi);
-}
-
-// largest m in 1..8 among the modes (shared, after ms is loaded)
-__device__ __forceinline__ int max_m(const int *ms, int K)
-{
-    int mm = 0;
-    for (int k = 0; k < K; ++k)
-        if (ms[k] >= 1 && ms[k] <= 8 && ms[k] > mm) mm = ms[k];
-    return mm;
 }
 
 __global__ void k_td2(double2 *out, const double *dataTime, const double *ts, const double *y, const double *c1,
@@ -97,7 +64,6 @@ __global__ void k_td2(double2 *out, const double *dataTime, const double *ts, co
     __shared__ int ms[kMaxTdModes];
     for (int k = threadIdx.x; k < K; k += blockDim.x) ms[k] = ms_in[k];
     __syncthreads();
-    const int mmax = max_m(ms, K);
     for (int b = blockIdx.y; b < B; b += gridDim.y) {
         // a binary's samples stop at max_length and its knot indices stay
         // inside its slot (the reference trusts its caller for both)
@@ -107,7 +73,7 @@ __global__ void k_td2(double2 *out, const double *dataTime, const double *ts, co
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += blockDim.x * gridDim.x) {
             const int ind = min(max(inds[(size_t)max_length * b + i], 0), old_length - 1);
             const double x = dataTime[i] - ts[(size_t)b * old_length + ind];
-            out[(size_t)b * data_length + i] = mode_sum(y, c1, c2, c3, base, (size_t)olh, ind, x, K, ms, mmax);
+            out[(size_t)b * data_length + i] = mode_sum(y, c1, c2, c3, base, (size_t)olh, ind, x, K, ms);
         }
     }
 }
@@ -122,11 +88,10 @@ __global__ void k_td1(double2 *out, const double *dataTime, const double *ts, co
     __shared__ int ms[kMaxTdModes];
     for (int k = threadIdx.x; k < K; k += blockDim.x) ms[k] = ms_in[k];
     __syncthreads();
-    const int mmax = max_m(ms, K);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += blockDim.x * gridDim.x) {
         const int ind = min(max(inds[i], 0), old_length - 1);
         const double x = dataTime[i + ind_start] - ts[ind];
-        out[(size_t)data_length + i] = mode_sum(y, c1, c2, c3, 0, (size_t)old_length, ind, x, K, ms, mmax);
+        out[(size_t)data_length + i] = mode_sum(y, c1, c2, c3, 0, (size_t)old_length, ind, x, K, ms);
     }
 }
 

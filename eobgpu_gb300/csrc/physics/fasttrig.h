@@ -95,10 +95,56 @@ __device__ __forceinline__ double unit_value(i64 v)
 static constexpr double kArgGammaH[7][EOB_ARG_GAMMA_N] = EOB_ARG_GAMMA_INIT;
 static constexpr double kArgGammaLowH[7][EOB_ARG_GAMMA_LOW_N] = EOB_ARG_GAMMA_LOW_INIT;
 
+#ifdef __CUDACC__
+// |x| >= 2^40, infinite or NaN
+__device__ __forceinline__ bool turns_refuse(double x)
+{
+    return (unsigned)(__double2hiint(x) & 0x7fffffff) >= 0x42700000u;
+}
+
+// The phase x of a sample, for sines and cosines of m x + add: m times the integer
+// phase is exact mod 1, and a rotation takes about 100 integer instructions, where
+// a complex product from one multiple to the next takes 4 FP64 ones (twice their
+// issue time) and a double product and sum with m converted 3.
+struct PhaseTurns {
+    u64 t;
+    double x;
+    bool large;
+    __device__ __forceinline__ explicit PhaseTurns(double phi) : x(phi)
+    {
+        large = turns_refuse(phi);
+        t = large ? 0ull : turns_of(phi);
+    }
+    __device__ __forceinline__ void fix(u64 turns, double *s, double *c) const
+    {
+        i64 sf, cf;
+        sincos_fix(turns, &sf, &cf);
+        *s = unit_value(sf);
+        *c = unit_value(cf);
+    }
+    __device__ __forceinline__ void wide(double arg, double *s, double *c) const
+    {
+        const double2 r = eob_sincos_large(arg);
+        *s = r.x;
+        *c = r.y;
+    }
+    __device__ __forceinline__ void multiple(int m, double *s, double *c) const
+    {
+        if (large) wide(m * x, s, c);
+        else fix((u64)(i64)m * t, s, c);
+    }
+    __device__ __forceinline__ void multiple(int m, double add, double *s, double *c) const
+    {
+        if (large || turns_refuse(add)) wide(fma((double)m, x, add), s, c);
+        else fix((u64)(i64)m * t + turns_of(add), s, c);
+    }
+};
+#endif
+
 EOB_HD void eob_sincos(double x, double *s, double *c)
 {
 #ifdef __CUDA_ARCH__
-    if ((unsigned)(__double2hiint(x) & 0x7fffffff) >= 0x42700000u) {  // |x| >= 2^40, inf, NaN
+    if (turns_refuse(x)) {
         const double2 r = eob_sincos_large(x);
         *s = r.x;
         *c = r.y;
