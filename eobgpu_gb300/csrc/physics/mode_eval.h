@@ -9,7 +9,8 @@
 // S of either parity) is formed once (ModeRow), and T_lm has no logarithm or
 // arctangent of its own.  With y = 2 k,
 //   |Gamma(l + 1 - i y)|^2 e^{pi y} = prod_{j<=l} (j^2 + y^2) 2 pi y / (1 - e^{-2 pi y})
-// (A&S 6.1.31, the closed form of the flux), and arg Gamma(l + 1 - i y) =
+// (A&S 6.1.31, the closed form of the flux; y = m y_1, so one exponential serves
+// every mode of a row, and one reciprocal square root its quotient's root), and arg Gamma(l + 1 - i y) =
 // -y P_l(y^2 / (l + 1)^2) with a polynomial per l (fasttrig.h) for
 // y <= 0.9 (l + 1), which every frequency of an inspiral meets (y < 2 m
 // Omega, Omega < 0.45).  Larger y go through the complex log Gamma: an
@@ -149,11 +150,23 @@ EOB_HD cdbl mode_eval_sums(const FacCoeffs &fc, int l, int m, double pre_re, dou
     return cmul(cmul(e, rf), cdbl{pre_re, pre_im});
 }
 
+// either zero, by its bits (a comparison of doubles takes an FP64 issue slot)
+EOB_HD bool is_zero(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (__double_as_longlong(x) << 1) == 0;
+#else
+    return x == 0.0;
+#endif
+}
+
 // What the modes of one trajectory point share.
 struct ModeRow {
-    double v, lv;       // omega^(1/3) and its logarithm
-    double Omega, Hreal;  // v^3, H_real
-    double vPhi;
+    double v, v2, lv;   // omega^(1/3), its square and its logarithm
+    double vh3;         // H_real v^3
+    double vh6, y1;     // its square and double
+    double E1;          // 1 - e^{-2 pi y1}
+    double vPhi, vPhi2, vPhi4;
     double Se, So;      // source terms of even and odd l + m
     double phi;
 };
@@ -162,14 +175,36 @@ EOB_HD ModeRow mode_row(double v, double Hreal, double vPhi, double pphi, double
 {
     ModeRow w;
     w.v = v;
+    w.v2 = v * v;
     w.lv = eob_log(v);
-    w.Omega = v * v * v;
-    w.Hreal = Hreal;
+    w.vh3 = Hreal * (w.v2 * v);
+    w.vh6 = w.vh3 * w.vh3;
+    w.y1 = 2.0 * w.vh3;
+    w.E1 = -eob_expm1_neg((2.0 * kPi) * w.y1);
     w.vPhi = vPhi;
+    w.vPhi2 = vPhi * vPhi;
+    w.vPhi4 = w.vPhi2 * w.vPhi2;
     w.Se = fma(fma(Hreal, Hreal, -1.0), inv2eta, 1.0);
     w.So = v * pphi;
     w.phi = phi;
     return w;
+}
+
+// 1 - e^{-m x} from E1 = 1 - e^{-x}: 1 - (1 - a)(1 - b) = a + b - a b, no cancellation
+EOB_HD double mode_expm(int m, double E1)
+{
+    if (m == 1) return E1;
+    const double E2 = fma(E1, -E1, E1 + E1);
+    if (m == 2) return E2;
+    if (m == 3) return fma(E2, -E1, E2 + E1);
+    const double E4 = fma(E2, -E2, E2 + E2);
+    double e = E4;
+    if (m == 8) e = fma(E4, -E4, E4 + E4);
+    else {
+        if (m & 2) e = fma(e, -E2, e + E2);
+        if (m & 1) e = fma(e, -E1, e + E1);
+    }
+    return e;
 }
 
 // What depends on (l, m) alone.
@@ -178,7 +213,7 @@ struct ModeConst {
     double tail;   // log(4 m / sqrt(e))
     double y0;     // (-1)^m Y_{l-eps}^m(pi/2, 0)
     double m, il;  // m, 1 / (l + 1)
-    double ifact;  // 1 / l!
+    double g[kLMax + 1];  // 2 pi prod_{j<=l} (1 + z / j^2), ascending in z
 };
 
 EOB_HD ModeConst mode_const(int l, int m)
@@ -189,8 +224,13 @@ EOB_HD ModeConst mode_const(int l, int m)
     c.y0 = ((m % 2) ? -1.0 : 1.0) * ylm_equator(l - (l + m) % 2, m);
     c.m = (double)m;
     c.il = 1.0 / (l + 1);
-    c.ifact = 1.0;
-    for (int q = 2; q <= l; ++q) c.ifact /= (double)q;
+    for (int q = 0; q <= kLMax; ++q) c.g[q] = (q == 0) ? 1.0 : 0.0;
+    double d = 2.0 * kPi;
+    for (int j = 1; j <= l; ++j) {  // prod (j^2 + z), integers, then over (l!)^2
+        for (int q = j; q >= 0; --q) c.g[q] = c.g[q] * (j * j) + (q > 0 ? c.g[q - 1] : 0.0);
+        d /= (double)(j * j);
+    }
+    for (int q = 0; q <= l; ++q) c.g[q] *= d;
     return c;
 }
 
@@ -201,11 +241,11 @@ EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, co
     if (eta > 0.25 && eta < 0.25 + 1e-4) eta = 0.25;
     const int i = lm_index(l, m);
     const int eps = (l + m) % 2;
-    const double v = w.v, v2 = v * v, vh3 = w.Hreal * w.Omega;
+    const double v = w.v, v2 = w.v2, vh3 = w.vh3;
     // delta_lm: the builder assigns vh^3, vh^6, vh^9 and v^5 only
     double delta = vh3 * fma(vh3, fma(vh3, fc.dvh[i][9], fc.dvh[i][6]), fc.dvh[i][3]);
     delta = fma(fc.dv[i][5], v2 * v2 * v, delta);
-    // rho_lm^l + f_lm (rho up to v^10, eulerlog parts at v^6, v^8, v^10; f from v^1 and v^3..v^6, l <= 5)
+    // rho_lm^l + f_lm (rho up to v^10, eulerlog parts at v^6, v^8, v^10; f for odd m <= 5, from v^1 and v^3..v^6)
     const double el = mc.elog + w.lv;
     const double c10 = fma(fc.rhol[i][10], el, fc.rho[i][10]), c8 = fma(fc.rhol[i][8], el, fc.rho[i][8]),
                  c6 = fma(fc.rhol[i][6], el, fc.rho[i][6]);
@@ -226,51 +266,63 @@ EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, co
         const double v4 = v2 * v2;
         rho = fma(h22_calib, v4 * v4 * v4, rho);
     }
-    double rpl = rho;
-    for (int q = 1; q < l; ++q) rpl *= rho;
-    double fr = 0.0;
-    if (l <= 5) {
+    const double rho2 = rho * rho;
+    double rpl = (l & 1) ? rho * rho2 : rho2;  // l = 2, 3
+    if (l >= 4) rpl *= rho2;
+    if (l >= 6) rpl *= rho2;
+    if (l >= 8) rpl *= rho2;
+    double fi = 0.0;
+    if ((m & 1) && l <= 5) {
         const double *f = fc.fre[i];
-        fr = v * fma(v2, fma(v, fma(v, fma(v, f[6], f[5]), f[4]), f[3]), f[1]);
+        const double fr = v * fma(v2, fma(v, fma(v, fma(v, f[6], f[5]), f[4]), f[3]), f[1]);
+        fi = fc.fim_vh6[i] * w.vh6;
+        rpl = (eta == 0.25) ? fr : rpl + fr;
+    } else if (m & 1) {
+        rpl = (eta == 0.25) ? 0.0 : rpl;
     }
-    const double fi = fc.fim_vh6[i] * vh3 * vh3;
-    cdbl rf = {rpl + fr, fi};
-    if (eta == 0.25 && (m % 2)) rf = {fr, fi};
-    // T_lm: its modulus and its phase without the logarithm's term
-    const double k = mc.m * w.Omega, hk = w.Hreal * k, y = 2.0 * hk;
+    // |T_lm|: sqrt(a / E), and its phase without the logarithm's term
+    const double y = mc.m * w.y1;
     double tmod, targ;
     const double q = y * mc.il, z = q * q;
     if (y >= 0.0 && z <= EOB_ARG_GAMMA_ZMAX) {
         targ = -y * (z <= EOB_ARG_GAMMA_ZLOW ? arg_gamma_over_y_low(l, z) : arg_gamma_over_y(l, z));
-        const double y2 = y * y, x = 2.0 * kPi * y;
-        double p = y2 + 1.0;
-        if (l >= 2) p *= y2 + 4.0;
-        if (l >= 3) p *= y2 + 9.0;
-        if (l >= 4) p *= y2 + 16.0;
-        if (l >= 5) p *= y2 + 25.0;
-        if (l >= 6) p *= y2 + 36.0;
-        if (l >= 7) p *= y2 + 49.0;
-        if (l >= 8) p *= y2 + 64.0;
+        const double y2 = y * y;
+        double a = mc.g[l];
+        for (int j = l - 1; j >= 0; --j) a = fma(a, y2, mc.g[j]);
+        a *= y;
 #ifdef __CUDA_ARCH__
-        const double t2 = x * eob_rcp(-eob_expm1_neg(x)) * p;
-        tmod = t2 * eob_rsqrt(t2) * mc.ifact;
+        tmod = a * eob_rsqrt(a * mode_expm(m, w.E1));
 #else
-        tmod = sqrt(x / -expm1(-x) * p) * mc.ifact;
+        tmod = sqrt(a / mode_expm(m, w.E1));
 #endif
     } else {
         double lgr;
         cloggamma_shifted(l + 1.0, -y, &lgr, &targ);
-        tmod = exp(kPi * hk + lgr) * mc.ifact;
+        tmod = exp(fma(0.5 * kPi, y, lgr)) * sqrt(mc.g[l] * (1.0 / (2.0 * kPi)));  // g[l] = 2 pi / (l!)^2
     }
     double phase = fma(y, fma(3.0, w.lv, mc.tail), targ) + delta;
     if (!derotate) phase -= mc.m * w.phi;
     double sp, cp;
     eob_sincos(phase, &sp, &cp);
-    double vpow = 1.0;
-    for (int j = 0; j < l + eps; ++j) vpow *= w.vPhi;
-    const double amp = tmod * (eps ? w.So : w.Se) * vpow * mc.y0;
-    const cdbl e = {amp * cp, amp * sp};
-    return cmul(cmul(e, rf), cdbl{pre_re, pre_im});
+    double amp = tmod * mc.y0 * (eps ? w.So : w.Se);
+    const int e = l + eps;
+    if (e & 1) amp *= w.vPhi;
+    if (e & 2) amp *= w.vPhi2;
+    if (e & 4) amp *= w.vPhi4;
+    if (e & 8) amp *= w.vPhi4 * w.vPhi4;
+    // times the Newtonian prefix, real or imaginary for the reference's own, and rpl + i fi
+    const bool real = is_zero(pre_im), imag = is_zero(pre_re);
+    if (real || imag) amp *= real ? pre_re : pre_im;
+    cdbl h;
+    if (l == 3 && m == 3) {  // the one mode with an imaginary part of f
+        h = cmul(cdbl{amp * cp, amp * sp}, cdbl{rpl, fi});
+    } else {
+        amp *= rpl;
+        h = cdbl{amp * cp, amp * sp};
+    }
+    if (real) return h;
+    if (imag) return cdbl{-h.im, h.re};
+    return cmul(h, cdbl{pre_re, pre_im});
 }
 
 // the same from the reference's arguments (vPhiInput = 1 / (omega_c^2 r^3))
