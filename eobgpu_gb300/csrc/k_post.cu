@@ -1,8 +1,8 @@
 // After the integrator: packing, multipoles on the trajectory and batched
 // not-a-knot splines.
 //
-//  k_scan_rows one block: per-binary row counts and waveform sample counts,
-//              exclusive scan (packed ragged layout).
+//  k_sample_counts  one thread per binary: waveform sample counts.
+//  k_scan_rows one block: exclusive scan of the row counts (packed ragged layout).
 //  k_modes     one thread per packed trajectory row: h_lm e^{i m phi} for the
 //              requested modes (get_hlms, eob/seobnrv4phm.py:2138-2221, and
 //              the de-rotation of compute_full_waveform, :2331).
@@ -33,8 +33,27 @@ __device__ int binary_npts(const double *tr, int L, double Mt, double dt)
     return (int)((t1 - t0) / dT) + 1;
 }
 
-// rows and uniform-grid sample counts per binary; packed row offsets
-__global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B, double dt)
+// Uniform-grid sample counts per binary.  A kernel of its own: three
+// divisions are 50 FP64 issue slots for each warp of binaries, which the scan's
+// one SM took 64 us for at 4096 binaries (8 us here and 7 us for the scan).
+__global__ void __launch_bounds__(128) k_sample_counts(Ws w, int B, double dt)
+{
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= B) return;
+    const int L = w.nsteps[b];
+    const int st = w.status[b];
+    int np = 0;
+    if (L >= 3 && !(st & (EOB_ST_NAN | EOB_ST_TRIES | EOB_ST_SHORT))) {
+        np = binary_npts(w.traj + (size_t)b * w.L.Lc * kTrajStride, L, w.bins[b].Mt, dt);
+        if (np < 1) np = 0;
+    } else {
+        w.status[b] = st | EOB_ST_SHORT;
+    }
+    w.npts[b] = np;
+}
+
+// packed row offsets
+__global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B)
 {
     __shared__ long long sm[34];
     const int tid = threadIdx.x;
@@ -42,20 +61,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B, double 
     const int b0 = tid * per;
     const int b1 = min(B, b0 + per);
     long long rows = 0;
-    for (int b = b0; b < b1; ++b) {
-        const int L = w.nsteps[b];
-        int st = w.status[b];
-        int np = 0;
-        if (L >= 3 && !(st & (EOB_ST_NAN | EOB_ST_TRIES | EOB_ST_SHORT))) {
-            np = binary_npts(w.traj + (size_t)b * w.L.Lc * kTrajStride, L, w.bins[b].Mt, dt);
-            if (np < 1) np = 0;
-        } else {
-            st |= EOB_ST_SHORT;
-            w.status[b] = st;
-        }
-        w.npts[b] = np;
-        rows += (np > 0) ? L : 0;
-    }
+    for (int b = b0; b < b1; ++b) rows += (w.npts[b] > 0) ? w.nsteps[b] : 0;
     long long total;
     long long ro = block_exclusive_scan<kScanThreads>(rows, sm, &total);
     for (int b = b0; b < b1; ++b) {
@@ -85,8 +91,8 @@ struct ModeArgs {
 // evaluations in one kernel cost the others their registers and half the
 // instruction cache (five modes, 4096 binaries, splines included: 5.8 ms
 // against 4.2 ms).  FP64 issue bounds both: five modes and the Hamiltonian
-// take 585 FP64 instructions a row in the closed form, 2427 by the sums on
-// every row (4096 binaries: 9.32 ms -> 2.25 + 0.47 ms; 1024 ragged binaries,
+// take 500 FP64 instructions a row in the closed form, 2427 by the sums on
+// every row (4096 binaries: 9.32 ms -> 1.92 + 0.47 ms; 1024 ragged binaries,
 // (2,2) alone: 0.77 -> 0.33 + 0.07 ms).
 __global__ void __launch_bounds__(128) k_modes(Ws w, int B, ModeArgs ma)
 {
@@ -237,7 +243,8 @@ cudaError_t launch_prepare_post(const Ws &w, const RunArgs &a, cudaStream_t s)
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    k_scan_rows<<<1, kScanThreads, 0, s>>>(w, a.B, a.dt);
+    k_sample_counts<<<(a.B + 127) / 128, 128, 0, s>>>(w, a.B, a.dt);
+    k_scan_rows<<<1, kScanThreads, 0, s>>>(w, a.B);
     ModeArgs ma;
     ma.K = a.K;
     for (int j = 0; j < kMaxModes; ++j) { ma.ells[j] = a.ells[j]; ma.mms[j] = a.mms[j]; }
