@@ -214,6 +214,7 @@ __device__ __forceinline__ void integrate_body(const IntArgs &a, X *xch_all, uns
     const unsigned gmask = (GW == 32) ? 0xffffffffu : (((1u << GW) - 1u) << (lane - sub));
     X *xch = nullptr;
     PairSync ps{0u, 0u, true};
+    const double md = (double)((lane & 7) + 1);
     QuadLane ql{};
     if constexpr (G == 128) ql = quad_lane(role, lane);
     if constexpr (kPair) {
@@ -355,7 +356,7 @@ __device__ __forceinline__ void integrate_body(const IntArgs &a, X *xch_all, uns
         // ------------------------------------------------ the one RHS per loop
         double kk[4];
         if constexpr (G == 1) eob_rhs(rec->ham, rec->flux, arg, kk);
-        else if constexpr (G == 64) eob_rhs_pair(rec->jets, rec->flux, arg, kk, lane, role, *xch, ps);
+        else if constexpr (G == 64) eob_rhs_pair(rec->jets, rec->flux, md, arg, kk, lane, role, *xch, ps);
         else if constexpr (G == 128) eob_rhs_quad(rec->jets, rec->flux, ql, arg, kk, lane, role, *xch, ps);
         else eob_rhs_group<G>(rec->jets, rec->flux, arg, kk, sub);
         if constexpr (kPair) {

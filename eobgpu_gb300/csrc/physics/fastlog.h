@@ -78,6 +78,20 @@ EOB_HD double bits_dbl(int64_t b)
 #endif
 }
 
+// (double)e, |e| < 2^20: on the device by integer operations (a conversion takes
+// an FP64 issue slot)
+EOB_HD double small_int(int e)
+{
+#ifdef __CUDA_ARCH__
+    const unsigned a = (unsigned)(e < 0 ? -e : e);
+    const int z = 31 - __clz((int)a);  // -1 for 0
+    const unsigned hi = ((unsigned)(1022 + z) << 20) + (a << (20 - z)) + ((unsigned)e & 0x80000000u);
+    return __hiloint2double(a ? (int)hi : 0, 0);
+#else
+    return (double)e;
+#endif
+}
+
 // log(x) for finite x >= 2^-1022 (the caller's arguments: r >= 1 and
 // v = omega^(1/3) in (0, 1)); other arguments go through eob_log below.
 EOB_HD double eob_log_normal(int64_t bits)
@@ -95,7 +109,7 @@ EOB_HD double eob_log_normal(int64_t bits)
     q = fma(q, z, 1.0 / 3.0);
     q = fma(q, z, -0.5);
     const double p = fma(z * z, q, z);
-    const double de = (double)e;
+    const double de = small_int(e);
     const double hi = fma(de, EOB_LN2_HI, t.thi);  // exact
     const double lo = fma(de, EOB_LN2_LO, t.tlo);
     return hi + (lo + p);

@@ -288,16 +288,22 @@ struct PartW {
     double W, Wu, Wp;
 };
 
-EOB_HD PartW comb_W(const Jet *jt, const CombB &b, double pr)
+EOB_HD double comb_W_q(const Jet *jt, double p2)  // 2 q_4 + 3 p_r^2 q_6 + 4 p_r^4 q_8
 {
-    const Jet q4 = jt[J_Q4], q6 = jt[J_Q6], q8 = jt[J_Q8];
+    return fma(p2, fma(4.0 * p2, jt[J_Q8].v, 3.0 * jt[J_Q6].v), 2.0 * jt[J_Q4].v);
+}
+
+EOB_HD PartW comb_W_of(const CombB &b, double pr, double q)
+{
     const double p2 = pr * pr;
     PartW o;
     o.W = fma(p2 * p2, b.qa, fma(p2, 1.0 + b.bnpv, 1.0));
     o.Wu = fma(p2 * p2, b.qad, p2 * b.bnpd);
-    o.Wp = 2.0 * pr * ((1.0 + b.bnpv) + p2 * fma(p2, fma(4.0 * p2, q8.v, 3.0 * q6.v), 2.0 * q4.v));
+    o.Wp = 2.0 * pr * fma(p2, q, 1.0 + b.bnpv);
     return o;
 }
+
+EOB_HD PartW comb_W(const Jet *jt, const CombB &b, double pr) { return comb_W_of(b, pr, comb_W_q(jt, pr * pr)); }
 
 // comb_W with dW/dp_r cut in two, for four warps: comb_W_b keeps its B_np
 // part 2 p_r (1 + B_np) and comb_Wp_q gives the rest,

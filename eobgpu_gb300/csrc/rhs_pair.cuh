@@ -12,10 +12,17 @@
 //   stage        role 0 (warp 2p)                 role 1 (warp 2p + 1)
 //   jets         log r, the log(r) parts          sqrt(u), the polynomial and
 //                                                 sqrt(u) parts (halves of the warp)
-//   combination  A(u), c(u)  -> even part         B_np, q  -> odd part
+//   combination  A(u), c(u)  -> W, even part      B_np, q, y_2/y_3  -> odd part
 //   H, flux      H and its gradient;              m factors (m x/(1-e^{-m x}), 4k^2),
-//                v = omega^(1/3), v_phi powers;   log v, y_2/y_3, 1/(8 pi nu); multipoles 32..34
-//                multipoles 0..31
+//                v = omega^(1/3), v_phi powers    log v
+//   multipoles   series parts of 0..31            m-factor parts of 0..31; 32..34
+//   (then the parts multiplied and summed by both warps)
+//
+// The split is by measured cycles of either warp between barriers (pair, 8 binaries):
+// jets 2.1 and 2.1 thousand, combination 2.0 and 1.9, even and odd part 2.3 and 2.3, H and
+// flux 3.6 and 3.9, multipoles 2.6 and 2.6, sum 1.1, the integrator 1.2 (with all of
+// multipoles 0..31 on role 0 that stage took 3.8, and the right-hand side 16.8
+// instead of 15.9).
 //
 // Values cross between the warps through shared memory at five pair
 // barriers per right-hand side (an mbarrier of 64 arrivals, waited on with a
@@ -37,13 +44,16 @@ constexpr int kPairMaxPolls = 1 << 28;                        // and at most thi
 // shared-memory exchange of one pair
 struct PairXchg {
     double jet[2][2][32];  // [part: 0 log, 1 poly+sqrt][v, d][lane]
-    double b[4][32];       // role 1 -> 0: bnpv, bnpd, qa, qad
+    double b[5][32];       // role 1 -> 0: bnpv, bnpd, qa, qad, the q part of dW/dp_r
     double ev[4][32];      // role 0 -> both: even part of H_eff and its derivatives
     double od[4][32];      // role 1 -> both: odd part
     double T[8], k4[8];    // role 1 -> 0: m factors, m = 1..8
-    double fl[13];         // v, log v (role 1 -> 0), v^12, S_even, S_odd, v_phi^(2e) e = 2..9 (role 0 -> 1)
-    double part[2];        // flux partial sums of the two warps
-    double aux[2];         // role 1 -> both: y_2 / y_3, 1 / (8 pi nu)
+    double fl[14];         // v, log v (role 1 -> 0), v^12, S_even^2, S_odd^2, v_phi^(2e) e = 2..9, v^2 (role 0 -> 1)
+    double ma[32];         // role 0 -> both: series parts of multipoles 0..31
+    double mb[32];         // role 1 -> both: their m-factor parts
+    double mt[3];          // role 1 -> both: multipoles 32..34
+    double aux[2];         // role 1 -> 0: y_2 / y_3, 1 / (8 pi nu)
+    double c[2];           // role 0 -> both: factors of the flux sum in dp_phi/dt and dp_r/dt
     double ham[3];         // role 0 -> both: dH/dr, dH/dp_r, dH/dL at the state
     unsigned long long slot;
 };
@@ -122,12 +132,21 @@ __device__ __forceinline__ double flux_warp_modes(const FluxTable &t, const Flux
 
 // k = f(y) for the binary of this pair; both warps call it with the same y
 // and return the same k.  role: 0 or 1; lane: 0..31.
-__device__ __forceinline__ void eob_rhs_pair(const HamJets &J, const FluxTable &t, const double y[4], double k[4],
-                                             int lane, int role, PairXchg &x, PairSync &ps)
+// md: (lane & 7) + 1 as a double (a conversion takes an FP64 issue slot).
+__device__ __forceinline__ void eob_rhs_pair(const HamJets &J, const FluxTable &t, double md, const double y[4],
+                                             double k[4], int lane, int role, PairXchg &x, PairSync &ps)
 {
     const double r = y[0], L = y[3];
     const int j = lane & 15;
-    const double u = eob_rcp(r);
+    double u, iL = 0.0;
+    if (role == 0) {
+        u = eob_rcp(r);
+    } else {
+        // 1 / y_3 on the upper lanes beside 1 / r
+        const double q = eob_rcp(lane < 16 ? r : L);
+        u = __shfl_sync(0xffffffffu, q, 0);
+        iL = __shfl_sync(0xffffffffu, q, 16);
+    }
 
     // ---- jets: role 0 the log(r) parts; role 1 the polynomial parts on
     // lanes 0..15 and the sqrt(u) parts on lanes 16..31
@@ -166,7 +185,7 @@ __device__ __forceinline__ void eob_rhs_pair(const HamJets &J, const FluxTable &
         b.bnpd = x.b[1][lane];
         b.qa = x.b[2][lane];
         b.qad = x.b[3][lane];
-        const HeffPart e = comb_even(jt, a, b, pr, L);
+        const HeffPart e = comb_even_parts({a.Av, a.Ad}, {a.cuv, a.cud}, comb_W_of(b, pr, x.b[4][lane]), L);
         x.ev[0][lane] = e.v;
         x.ev[1][lane] = e.du;
         x.ev[2][lane] = e.dp;
@@ -178,8 +197,9 @@ __device__ __forceinline__ void eob_rhs_pair(const HamJets &J, const FluxTable &
         x.b[1][lane] = b.bnpd;
         x.b[2][lane] = b.qa;
         x.b[3][lane] = b.qad;
+        x.b[4][lane] = comb_W_q(jt, pr * pr);
         if (lane == 0) {
-            x.aux[0] = y[2] * eob_rcp(y[3]);
+            x.aux[0] = y[2] * iL;
             x.aux[1] = J.inv8pinu;
         }
         pair_sync(ps);  // 2
@@ -200,7 +220,6 @@ __device__ __forceinline__ void eob_rhs_pair(const HamJets &J, const FluxTable &
     od.dp = x.od[2][lane];
     od.dL = x.od[3][lane];
     // ---- H and the flux set-up
-    double part;
     if (role == 0) {
         const HamPart hp = comb_final(J, u, ev, od);
         const double Hreal = __shfl_sync(0xffffffffu, hp.Hreal, 0);
@@ -220,22 +239,29 @@ __device__ __forceinline__ void eob_rhs_pair(const HamJets &J, const FluxTable &
         if (lane == 0) {
             x.fl[0] = f.v;
             x.fl[2] = f.v12;
-            x.fl[3] = f.Se;
-            x.fl[4] = f.Sodd;
+            x.fl[3] = f.S2e;
+            x.fl[4] = f.S2o;
+            x.fl[13] = f.v2;
 #pragma unroll
             for (int q = 0; q < 8; ++q) x.fl[5 + q] = f.vp[q];
         }
         pair_sync(ps);  // 4: FluxLane, log v and m factors
         f.lv = x.fl[1];
-        part = flux_warp_modes<0>(t, f, x, lane);
+        x.ma[lane] = flux_mode_a<kFluxDegSorted[0], flux_lmax(0, 32), flux_lmin(0, 32)>(t, kFluxOrder[lane], f);
+        // F / omega = total c1 with F = total omega^2 / (8 pi) / nu, and
+        // (y_2 / y_3) F / omega = total c2
+        const double c1 = omega * x.aux[1], c2 = x.aux[0] * c1;
+        if (lane == 0) {
+            x.c[0] = c1;
+            x.c[1] = c2;
+        }
     } else {
         // this warp needs H_real omega and omega, not the whole combination:
         // with D = dH_eff/dL, H_real omega = M^2 D exactly (H_real = M s,
         // omega = M D / s), and omega = M D / s with s from the same square root
         const double D = x.ev[3][0] + x.od[3][0];
         const double hw = J.M2 * D;
-        double Tm, k4m;
-        flux_m_factors((lane & 7) + 1, 4.0 * kPi * hw, hw, &Tm, &k4m);
+        const double Tm = flux_m_factor_T(md, 4.0 * kPi * hw), k4m = flux_m_factor_k4(md, hw);
         if (lane < 8) {
             x.T[lane] = Tm;
             x.k4[lane] = k4m;
@@ -250,30 +276,31 @@ __device__ __forceinline__ void eob_rhs_pair(const HamJets &J, const FluxTable &
         pair_sync(ps);  // 4
         FluxLane f;
         f.v = x.fl[0];
-        f.v2 = f.v * f.v;
+        f.v2 = x.fl[13];
         f.lv = x.fl[1];
         f.v12 = x.fl[2];
-        f.Se = x.fl[3];
-        f.Sodd = x.fl[4];
-        f.S2e = f.Se * f.Se;
-        f.S2o = f.Sodd * f.Sodd;
+        f.S2e = x.fl[3];
+        f.S2o = x.fl[4];
+        f.Se = 0.0;
+        f.Sodd = 0.0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) f.vp[q] = x.fl[5 + q];
-        part = flux_warp_modes<32>(t, f, x, lane);
+        const int i = kFluxOrder[lane], m = lm_packed(i) & 15;
+        x.mb[lane] = flux_mode_b<flux_lmax(0, 32)>(t, i, x.T[m - 1], x.k4[m - 1]);
+        const double last = flux_warp_modes<32>(t, f, x, lane);
+        if (lane < 3) x.mt[lane] = last;
     }
-    // F / omega = total c1 with F = total omega^2 / (8 pi) / nu, and
-    // (y_2 / y_3) F / omega = total c2, beside the reduction
-    const double omega = x.ham[2];
-    const double c1 = omega * x.aux[1], c2 = x.aux[0] * c1;
+    pair_sync(ps);  // 5: the multipoles' parts
+    // the sum of the products, by both warps on the same shared values (the
+    // same bits on every lane: addition commutes)
+    double part = __dmul_rn(x.mb[lane], x.ma[lane]);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-    if (lane == 0) x.part[role] = part;
-    pair_sync(ps);  // 5: flux partial sums
-    const double total = x.part[0] + x.part[1];
+    const double total = part + ((x.mt[0] + x.mt[2]) + x.mt[1]);
     k[0] = x.ham[1];
-    k[1] = omega;
-    k[2] = -fma(c2, total, x.ham[0]);
-    k[3] = -(total * c1);
+    k[1] = x.ham[2];
+    k[2] = -fma(x.c[1], total, x.ham[0]);
+    k[3] = -(total * x.c[0]);
 }
 
 }  // namespace eob
