@@ -38,21 +38,28 @@ __device__ __forceinline__ double cubic(const double *y, const double *c1, const
 // bounds it (88 %): two modes take 24 FP64 instructions a sample, 72 with the
 // library's sincos and products for the powers of x, 28 with integer sincos and
 // complex products from one multiple to the next (128 binaries, two modes, 32768
-// samples: 0.36, 0.18 and 0.145 ms).
+// samples: 0.36, 0.18 and 0.143 ms).
 __device__ __forceinline__ double2 mode_sum(const double *y, const double *c1, const double *c2, const double *c3,
                                             size_t base, size_t stride, int ind, double x, int K, const int *ms)
 {
-    // one mode: the phase m phi is rounded once, as a single series' caller would
     const double phi = cubic(y, c1, c2, c3, base + 2 * (size_t)K * stride + ind, x);
-    const eob::PhaseTurns phase(K == 1 ? ms[0] * phi : phi);
-    double hr = 0.0, hi = 0.0, c = 0.0, s = 0.0;
-    for (int k = 0; k < K; ++k) {
-        if (k == 0 || ms[k] != ms[k - 1]) phase.multiple(K == 1 ? 1 : ms[k], &s, &c);
+    double hr = 0.0, hi = 0.0, c, s;
+    auto add = [&](int k) {
         const double re = cubic(y, c1, c2, c3, base + (size_t)k * stride + ind, x);
         const double im = cubic(y, c1, c2, c3, base + (size_t)(K + k) * stride + ind, x);
         // (re + i im)(c - i s)
         hr = fma(re, c, fma(im, s, hr));
         hi = fma(im, c, fma(-re, s, hi));
+    };
+    if (K == 1) {  // the phase m phi rounded once, as a single series' caller would
+        eob::eob_sincos(ms[0] * phi, &s, &c);
+        add(0);
+        return make_double2(hr, hi);
+    }
+    const eob::PhaseTurns phase(phi);
+    for (int k = 0; k < K; ++k) {
+        if (k == 0 || ms[k] != ms[k - 1]) phase.multiple(ms[k], &s, &c);
+        add(k);
     }
     return make_double2(hr, hi);
 }
