@@ -75,9 +75,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B)
     }
 }
 
-// rows closer than this to a neighbour [M] keep the log-Gamma sums (mode_eval.h); the
-// fine pass steps by 0.05 and halves
-constexpr double kCloseRows = 0.04;
+// rows closer than this to a neighbour [M] keep the log-Gamma sums (mode_eval.h): the
+// fine pass steps by 0.05 and halves; the main pass's steps are above 0.2 but at
+// its end
+constexpr double kCloseRows = 0.2;
 
 struct ModeArgs {
     int K;

@@ -1,5 +1,5 @@
 """The fused path's multipoles on every trajectory row -- the closed form on
-ordinary rows, the log-Gamma sums on rows closer than 0.04 M -- against the
+ordinary rows, the log-Gamma sums on the fine pass's -- against the
 reference-shaped compute_hlms on the same rows, rotated by e^{i m phi}: one
 function, within 1e-12 of each mode's peak (its evaluations round at 2e-14, the
 rotation at eps of phases up to 1e3 rad, 2e-13)."""
