@@ -531,8 +531,9 @@ def run_op(args, local):
     samples or 2^16 + 1 frequency bins): --op tdinterp2 (mode synthesis on the
     uniform grid, TD2) or --op fd_lnl (frequency-domain likelihood partials,
     three detectors).  Reports the kernel time, algorithmic bytes and the
-    fraction of the measured HBM bandwidth; both kernels evaluate one FP64
-    sincos per output (per mode for TD2), so they are FP64-issue bound."""
+    fraction of the measured HBM bandwidth.  TD2 is bound by FP64 issue (its
+    sines and cosines run on the integer units), the likelihoods by integer
+    issue."""
     import torch
     from eobgpu_gb300.eob import pytdinterp
     device = torch.device(f"cuda:{local}")
@@ -622,7 +623,7 @@ def run_op(args, local):
     gbs = byts / (t / 1e3) / 1e9
     from eobgpu_gb300 import _lib
     pk = fp64_peak_tflops(_lib.load(), device)
-    roof = {"bound": "fp64", "achieved": None, "peak": pk, "unit": "TFLOP/s", "frac": None, "traffic": None,
+    roof = {"bound": "fp64" if args.op == "tdinterp2" else "integer issue", "achieved": None, "peak": pk, "unit": "TFLOP/s", "frac": None, "traffic": None,
             "work": work, "peak_source": "measured live: FP64 DFMA probe (eob_fp64_probe), burst",
             "hbm": {"achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                     "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)"}}
@@ -755,7 +756,7 @@ def run_serving(args, ws, rank, local):
                 "e2e": {"value": value, "unit": "evals/s", "h2d_bytes_per_step": int(nbin / ws * 40),
                         "d2h_bytes_per_step": int(nbin / ws * 12)},
                 "latency_ms": sv["replay"]["latency_ms"], "serving": sv,
-                "gpu_launches": int(8 * res["batches"]), "roofline": None, "cpu_baseline": None,
+                "gpu_launches": int(11 * res["batches"]), "roofline": None, "cpu_baseline": None,
                 "clocks": sv.get("clocks"), "status_ok": sv["replay"]["status_ok"]}
         if args.accuracy_sample > 0:
             cfg = workload.CONFIGS[1]
@@ -1053,7 +1054,9 @@ def main():
             t, _ = cpu_time(sample, cfg, data, amp, args.max_steps, cores)
             cpu_base = {"value": len(sample) / t, "unit": "evals/s", "cores": cores, "kind": "port",
                         "sample": f"{len(sample)} of {B} binaries (every {max(1, B // args.cpu_sample)}th)"}
-        launches_per_step = 8  # setup, integrate, scan_rows, modes, spline, scan_chunks, synth, finalize
+        # setup, integrate, sample_counts, scan_rows, modes, modes_close, splines (long, short), scan_chunks, synth,
+        # finalize
+        launches_per_step = 11
         line = {"metric": METRIC, "value": value, "unit": "evals/s", "n_gpus": ws, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": t_dev / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None,

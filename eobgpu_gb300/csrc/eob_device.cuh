@@ -111,7 +111,7 @@ struct Ws {
     double *traj;
     int *nsteps, *status;
     int *rhs;                   // right-hand sides evaluated for each binary (both passes, all attempts)
-    unsigned long long *queue;  // [0] work queue, [1] total rows, [2] total chunks, [3] sum data^2 (double bits),
+    unsigned long long *queue;  // [0] work queue, [1] total rows, [2] total chunks, [3] unused,
                                 // [4] RHS evaluations for binaries, [5] RHS evaluations incl. idle lanes,
                                 // [6] 1 if the spline build wrote FP32 copies (mixed precision)
     long long *row_off, *chunk_off;

@@ -90,11 +90,10 @@ struct ModeArgs {
 // Rows closer than kCloseRows to a neighbour are listed (in the spline
 // scratch, which is free until the splines) for k_modes_close: the two
 // evaluations in one kernel cost the others their registers and half the
-// instruction cache (five modes, 4096 binaries, splines included: 5.8 ms
-// against 4.2 ms).  FP64 issue bounds both: five modes and the Hamiltonian
-// take 500 FP64 instructions a row in the closed form, 2427 by the sums on
-// every row (4096 binaries: 9.32 ms -> 1.92 + 0.47 ms; 1024 ragged binaries,
-// (2,2) alone: 0.77 -> 0.33 + 0.07 ms).
+// instruction cache.  FP64 issue bounds both: five modes and the Hamiltonian
+// take 500 FP64 instructions a row in the closed form, 2550 by the sums (4096
+// binaries, 2.1 M rows, 4 in 10 listed: 9.32 ms with the sums on every row -> 1.13 + 4.39 ms;
+// 1024 ragged binaries, (2,2) alone: 0.77 -> 0.23 + 0.34 ms).
 __global__ void __launch_bounds__(128) k_modes(Ws w, int B, ModeArgs ma)
 {
     const long long R = (long long)w.queue[1];

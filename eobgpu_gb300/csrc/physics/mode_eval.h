@@ -20,12 +20,13 @@
 // used.
 //
 // mode_eval_sums is the evaluation by the sums of log Gamma throughout.  They
-// cancel from ~30 to order one and leave 4e-15 of rounding in the modulus
-// (rms against 40 digits; 1.5e-15 the closed form).  On rows closer than the
-// fine pass's step of 0.05 M (steps halved at the plunge) the third differences
-// of the spline amplify rounding by 1e7 and more, so that c3 there is rounding; k_modes keeps
-// those rows (3 in 100) on the sums, so that their tables do not move with the
-// evaluation of the others.
+// cancel from ~30 to order one and leave 4e-15 of rounding in the modulus (rms
+// against 40 digits; 1.5e-15 the closed form).  On the rows of the fine pass (0.05 M
+// apart and less) the third differences of the spline amplify rounding by 1e4
+// to 1e8, so that their c3 is rounding: 4e-15 of the modulus are up to 6e-8 of
+// its norm.  k_modes leaves those rows (4 in 10) to the sums, so that the tables
+// do not move with the evaluation of the others; a change of one last bit in the
+// sums (an arctangent by its series, logarithms shared by the modes) moves them too.
 // With derotate = true the result is multiplied by e^{i m phi}: the
 // e^{-i m phi} of the spherical harmonic is simply not applied, which is what
 // the spline inputs of the synthesis need (eob/seobnrv4phm.py:2331).

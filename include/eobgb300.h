@@ -55,7 +55,8 @@ typedef struct eob_options {
     int lanes_per_binary;   /* integrator lanes per binary: 1, 2, 4, 8, 16, 32, 64 (two warps on two SM
                                sub-partitions) or 128 (four warps, one per sub-partition of an SM);
                                0 = chosen from the batch size */
-    int spline_tile;        /* spline build: series (one warp each) per block, 1..8 (0 = default 4) */
+    int spline_tile;        /* spline build: series per block, which factorises its binary's matrix once
+                               (0 = all of them, or fewer while the batch leaves SMs idle) */
     int head_quads;         /* with warp pairs or groups of 8, 16 or 32 lanes: the head_quads longest
                                binaries (first in `order`) on four warps each, concurrently with the rest
                                (-1 = chosen from the batch: with warp pairs min(B / 64, 16), otherwise
@@ -304,7 +305,8 @@ int eob_detector_response(const double *ra, const double *dec, const double *psi
  * / psd_c(f) with data[c][N/2 + 1] (complex), psd[c][N/2 + 1], Fplus, Fcross,
  * time_shift[c * B + b] (the all_in_one_likelihood partials,
  * src/interpolate.cu:551-627, summed).  nch <= 8.  scratch: device memory of
- * eob_fd_lnl_scratch_bytes(B, N) bytes (block partials and 1/psd). */
+ * eob_fd_lnl_scratch_bytes(B, N) bytes (block partials, the data and the detectors'
+ * phases as integers). */
 size_t eob_fd_lnl_scratch_bytes(int B, int N);
 int eob_fd_lnl_from_fft(const double *H, int N, int start_ind, const double *data, const double *psd,
                         const double *Fplus, const double *Fcross, const double *time_shift, double df, int B, int nch,
