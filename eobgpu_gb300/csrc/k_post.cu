@@ -125,7 +125,9 @@ __global__ void __launch_bounds__(128) k_modes(Ws w, int B, ModeArgs ma)
         for (int j = 0; j < ma.K; ++j) {
             const int l = ma.ells[j], m = ma.mms[j];
             const int li = lm_index(l, m);
-            const cdbl hl = mode_term(w.fac[b], l, m, ma.mc[j], mr, rec.pre_re[li], rec.pre_im[li], rec.nu, 0.0, true);
+            // set-up builds every table with use_hm = 1
+            const cdbl hl = mode_term<true>(w.fac[b], l, m, ma.mc[j], mr, rec.pre_re[li], rec.pre_im[li], rec.nu, 0.0,
+                                            true);
             w.ys[(size_t)(1 + 2 * j) * Rc + r] = hl.re;
             w.ys[(size_t)(2 + 2 * j) * Rc + r] = hl.im;
         }

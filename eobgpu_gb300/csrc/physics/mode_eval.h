@@ -19,7 +19,7 @@
 // logarithm does not matter.  The reference's SciPy-derived loggamma is not
 // used.
 //
-// mode_eval_sums is the evaluation by the sums of log Gamma throughout.  They
+// mode_eval_sums is the evaluation by the sums of log Gamma throughout, for tables of use_hm = 1.  They
 // cancel from ~30 to order one and leave 4e-15 of rounding in the modulus (rms
 // against 40 digits; 1.5e-15 the closed form).  On the rows of the fine pass (0.05 M
 // apart and less) the third differences of the spline amplify rounding by 1e4
@@ -235,7 +235,11 @@ EOB_HD ModeConst mode_const(int l, int m)
     return c;
 }
 
-// h_lm (or h_lm e^{i m phi} when derotate). i = lm_index(l, m).
+// h_lm (or h_lm e^{i m phi} when derotate). i = lm_index(l, m).  HM: the table
+// was built with use_hm = 1, which leaves the odd powers of v in rho_lm (and the
+// logarithm beside v^7) to a few modes; otherwise a = tplspin brings them to
+// most modes and the whole series is summed.
+template <bool HM>
 EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, const ModeRow &w, double pre_re,
                       double pre_im, double eta, double h22_calib, bool derotate)
 {
@@ -246,16 +250,18 @@ EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, co
     // delta_lm: the builder assigns vh^3, vh^6, vh^9 and v^5 only
     double delta = vh3 * fma(vh3, fma(vh3, fc.dvh[i][9], fc.dvh[i][6]), fc.dvh[i][3]);
     delta = fma(fc.dv[i][5], v2 * v2 * v, delta);
-    // rho_lm^l + f_lm (rho up to v^10, eulerlog parts at v^6, v^8, v^10; f for odd m <= 5, from v^1 and v^3..v^6)
+    // rho_lm^l + f_lm (rho up to v^10, eulerlog parts at v^6, v^8, v^10 and, without HM, v^7; f for odd m <= 5, from
+    // v^1 and v^3..v^6)
     const double el = mc.elog + w.lv;
     const double c10 = fma(fc.rhol[i][10], el, fc.rho[i][10]), c8 = fma(fc.rhol[i][8], el, fc.rho[i][8]),
                  c6 = fma(fc.rhol[i][6], el, fc.rho[i][6]);
     double rho;
-    if ((l == m && (l & 1) == 0) || (l == 3 && m == 2) || (l == 4 && m == 2)) {
+    if (!HM || (l == m && (l & 1) == 0) || (l == 3 && m == 2) || (l == 4 && m == 2)) {
         // odd powers too
         const double *c = fc.rho[i];
+        const double c7 = HM ? c[7] : fma(fc.rhol[i][7], el, c[7]);
         rho = fma(fma(c10, v, c[9]), v, c8);
-        rho = fma(fma(rho, v, c[7]), v, c6);
+        rho = fma(fma(rho, v, c7), v, c6);
         rho = fma(fma(rho, v, c[5]), v, c[4]);
         rho = fma(fma(rho, v, c[3]), v, c[2]);
         rho = fma(rho, v, c[1]) * v;
@@ -326,13 +332,13 @@ EOB_HD cdbl mode_term(const FacCoeffs &fc, int l, int m, const ModeConst &mc, co
     return cmul(h, cdbl{pre_re, pre_im});
 }
 
-// the same from the reference's arguments (vPhiInput = 1 / (omega_c^2 r^3))
+// the same from the reference's arguments (vPhiInput = 1 / (omega_c^2 r^3)), for a table of either use_hm
 EOB_HD cdbl mode_eval(const FacCoeffs &fc, int l, int m, double pre_re, double pre_im, double eta, double r, double phi,
                       double pphi, double v, double Hreal, double vPhiInput, double h22_calib, bool derotate)
 {
     const double e4 = (eta > 0.25 && eta < 0.25 + 1e-4) ? 0.25 : eta;
     const ModeRow w = mode_row(v, Hreal, r * cbrt(vPhiInput) * (v * v * v), pphi, 0.5 / e4, phi);
-    return mode_term(fc, l, m, mode_const(l, m), w, pre_re, pre_im, eta, h22_calib, derotate);
+    return mode_term<false>(fc, l, m, mode_const(l, m), w, pre_re, pre_im, eta, h22_calib, derotate);
 }
 
 }  // namespace eob
