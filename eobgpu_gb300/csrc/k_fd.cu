@@ -208,13 +208,14 @@ int eob_detector_response(const double *ra, const double *dec, const double *psi
 }
 
 // block partials of every binary, then the data with 1 / S_n and the per-binary
-// constants of up to kFdMaxChannels detectors (256-byte aligned)
+// constants of up to kFdMaxChannels detectors.  FdData is loaded 16 bytes at a time and
+// starts at the next multiple of its alignment: the scratch itself may be aligned to 8 only
 size_t eob_fd_lnl_scratch_bytes(int B, int N)
 {
     if (B < 1 || N < 2) return 0;
     const long long nblk = ((long long)(N / 2 + 1) + kFdBins - 1) / kFdBins;
     const size_t part = ((size_t)(nblk * B) * sizeof(double) + 255) & ~(size_t)255;
-    return part + (size_t)kFdMaxChannels * ((size_t)(N / 2 + 1) * sizeof(FdData) + (size_t)B * sizeof(FdDetector));
+    return part + alignof(FdData) + (size_t)kFdMaxChannels * ((size_t)(N / 2 + 1) * sizeof(FdData) + (size_t)B * sizeof(FdDetector));
 }
 
 int eob_fd_lnl_from_fft(const double *H, int N, int start_ind, const double *data, const double *psd,
@@ -227,7 +228,7 @@ int eob_fd_lnl_from_fft(const double *H, int N, int start_ind, const double *dat
     const int nblk = (N / 2 + 1 + kFdBins - 1) / kFdBins;
     double *partial = (double *)scratch;
     const size_t part = ((size_t)nblk * (size_t)B * sizeof(double) + 255) & ~(size_t)255;
-    FdData *fixed = (FdData *)((char *)scratch + part);
+    FdData *fixed = (FdData *)(((uintptr_t)scratch + part + alignof(FdData) - 1) & ~(uintptr_t)(alignof(FdData) - 1));
     const long long nbin = (long long)nch * (N / 2 + 1);
     k_fd_data<<<blocks_for(nbin, 128), 128, 0, stream>>>((const double2 *)data, psd, nbin, fixed);
     if (cudaGetLastError() != cudaSuccess) return EOB_E_CUDA;
