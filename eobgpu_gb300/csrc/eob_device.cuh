@@ -117,13 +117,15 @@ struct Ws {
     long long *row_off, *chunk_off;
     int *npts;
     double *tin, *ys, *cA, *cB, *cC, *cD, *partial;
-    float *f32;    // mixed precision: (y, c1, c2, c3) of the mode series, [2K][rows][4]
+    float *f32;    // mixed precision: (y, c1, c2, c3) of the mode series, [2K][rows][4]; a float4 where f32_vec()
     float *dataf;  // mixed precision: data in FP32
     // merger-ringdown section (null when the workspace has none)
     double *imr_ys, *imr_cA, *imr_cB, *imr_cC, *imr_cD;  // series 0: r, 1: p_r
     ImrRec *imr_rec;                                     // [b * Kc + q]
     ImrBin *imr_bin;
     WsLayout L;
+    // the workspace may be aligned to 8 bytes only; its vector loads are taken where it is to 16
+    EOB_HD bool f32_vec() const { return (reinterpret_cast<uintptr_t>(f32) & 15) == 0; }
 };
 
 inline Ws ws_views(void *base, const WsLayout &L)

@@ -201,8 +201,16 @@ struct PackedSplines {
         f.c3[i] = c3;
         if (mixed && s >= 1 && s < nmain) {
             // FP32 copies of the amplitude series for the mixed-precision synthesis
-            reinterpret_cast<float4 *>(w.f32)[(size_t)(s - 1) * Rc + base + i] =
-                make_float4((float)f.y[i], (float)c1, (float)c2, (float)c3);
+            const float4 v = make_float4((float)f.y[i], (float)c1, (float)c2, (float)c3);
+            float *o = w.f32 + 4 * ((size_t)(s - 1) * Rc + base + i);
+            if (w.f32_vec()) {
+                *reinterpret_cast<float4 *>(o) = v;
+            } else {
+                o[0] = v.x;
+                o[1] = v.y;
+                o[2] = v.z;
+                o[3] = v.w;
+            }
         }
     }
     __device__ void put_last(int b, int s, int i, const SplineSeries &f, double, double, double) const
