@@ -114,7 +114,8 @@ struct Ws {
     unsigned long long *queue;  // [0] work queue, [1] total rows, [2] total chunks, [3] unused,
                                 // [4] RHS evaluations for binaries, [5] RHS evaluations incl. idle lanes,
                                 // [6] 1 if the spline build wrote FP32 copies (mixed precision)
-    long long *row_off, *chunk_off;
+    long long *row_off;
+    long long *chunk_off;       // until the synthesis: the splines' work order, as ints
     int *npts;
     double *tin, *ys, *cA, *cB, *cC, *cD, *partial;
     float *f32;    // mixed precision: (y, c1, c2, c3) of the mode series, [2K][rows][4]; a float4 where f32_vec()

@@ -52,10 +52,16 @@ __global__ void __launch_bounds__(128) k_sample_counts(Ws w, int B, double dt)
     w.npts[b] = np;
 }
 
-// packed row offsets
+// packed row offsets, and the splines' work order, longest binaries first in steps
+// of 64 rows (to chunk_off, which the synthesis fills later).  The caller's `order` is the
+// integrator's alone and need not name every binary; in batch order the long splines
+// of 1024 ragged binaries end 22 us later.
+constexpr int kLengthSteps = 64;
+
 __global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B)
 {
     __shared__ long long sm[34];
+    __shared__ int place[kLengthSteps];
     const int tid = threadIdx.x;
     const int per = (B + kScanThreads - 1) / kScanThreads;
     const int b0 = tid * per;
@@ -73,6 +79,22 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_rows(Ws w, int B)
         w.queue[1] = (unsigned long long)total;
         *(unsigned long long *)w.partial = 0;  // k_modes counts its close rows here
     }
+    if (tid < kLengthSteps) place[tid] = 0;
+    __syncthreads();
+    auto step = [&](int b) { return kLengthSteps - 1 - max(0, min(w.nsteps[b] / 64, kLengthSteps - 1)); };
+    for (int b = b0; b < b1; ++b) atomicAdd(&place[step(b)], 1);
+    __syncthreads();
+    if (tid == 0) {
+        int at = 0;
+        for (int q = 0; q < kLengthSteps; ++q) {
+            const int n = place[q];
+            place[q] = at;
+            at += n;
+        }
+    }
+    __syncthreads();
+    int *order = reinterpret_cast<int *>(w.chunk_off);
+    for (int b = b0; b < b1; ++b) order[atomicAdd(&place[step(b)], 1)] = b;
 }
 
 // rows closer than this to a neighbour [M] keep the log-Gamma sums (mode_eval.h): the
@@ -222,8 +244,8 @@ struct PackedSplines {
 constexpr int kSplineThreads = 64, kSplineChunk = 9, kSplineShort = kSplineThreads * kSplineChunk;
 constexpr int kSplineLongThreads = 256;
 
-// One block per binary and group of `per` series, in the caller's queue order
-// (longest first).  NT = 64 threads of up to 9 rows: 576 rows a tile, which most
+// One block per binary and group of `per` series, long binaries first.  NT = 64 threads
+// of up to 9 rows: 576 rows a tile, which most
 // trajectories fit; 128 threads of 5 rows would spend a quarter more FP64 issue
 // slots on the scans, and chunks of 13 rows hold their factors in 250 registers (four
 // blocks on an SM; six with the 168 of a bound of five, which spills 100 bytes).
@@ -234,13 +256,13 @@ constexpr int kSplineLongThreads = 256;
 // 13 rows for all, 0.26 so; 4096 binaries, 11 series, 520 rows: 4.67, 1.19
 // and 1.08 + 0.03 ms (79 % of the FP64 issue slots).
 template <int NT>
-__global__ void __launch_bounds__(NT, NT == 64 ? 5 : 1) k_spline(Ws w, const int *order, int nsubs, int nmain, int per, int mixed)
+__global__ void __launch_bounds__(NT, NT == 64 ? 5 : 1) k_spline(Ws w, int nsubs, int nmain, int per, int mixed)
 {
     using Block = SplineBlock<1, NT, kSplineChunk>;
     extern __shared__ __align__(16) char smem[];
     typename Block::Smem &sm = *reinterpret_cast<typename Block::Smem *>(smem);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) w.queue[6] = (unsigned long long)mixed;
-    const int b = order ? order[blockIdx.x] : blockIdx.x;
+    const int b = reinterpret_cast<const int *>(w.chunk_off)[blockIdx.x];  // k_scan_rows
     const int n = w.npts[b] > 0 ? w.nsteps[b] : 0;
     if ((n > kSplineShort) != (NT > kSplineThreads)) return;
     const PackedSplines acc{w, n, nmain, (size_t)w.row_off[b], (size_t)w.L.Bc * (size_t)w.L.Lc, mixed != 0};
@@ -279,9 +301,9 @@ cudaError_t launch_prepare_post(const Ws &w, const RunArgs &a, cudaStream_t s)
         const cudaError_t e = cudaFuncSetAttribute(k_spline<kSplineLongThreads>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Long));
         if (e != cudaSuccess) return e;
-        k_spline<kSplineLongThreads><<<grid, kSplineLongThreads, sizeof(Long), s>>>(w, a.order, nsubs, nmain, per, mixed);
+        k_spline<kSplineLongThreads><<<grid, kSplineLongThreads, sizeof(Long), s>>>(w, nsubs, nmain, per, mixed);
     }
-    k_spline<kSplineThreads><<<grid, kSplineThreads, sizeof(Short), s>>>(w, a.order, nsubs, nmain, per, mixed);
+    k_spline<kSplineThreads><<<grid, kSplineThreads, sizeof(Short), s>>>(w, nsubs, nmain, per, mixed);
     return cudaGetLastError();
 }
 
