@@ -18,10 +18,12 @@ namespace {
 constexpr int kTPB = 128;
 inline int nblk(long long n) { return (int)((n + kTPB - 1) / kTPB); }
 
+template <bool FIXED = false>
 __device__ void ham_of_add(HamCoeffs *h, const double *add, int n, int i)
 {
-    ham_coeffs_build(h, add[i], add[(size_t)n + i], add[2 * (size_t)n + i], add[3 * (size_t)n + i],
-                     add[5 * (size_t)n + i], add[6 * (size_t)n + i], add[7 * (size_t)n + i], add[8 * (size_t)n + i]);
+    ham_coeffs_build<FIXED>(h, add[i], add[(size_t)n + i], add[2 * (size_t)n + i], add[3 * (size_t)n + i],
+                            add[5 * (size_t)n + i], add[6 * (size_t)n + i], add[7 * (size_t)n + i],
+                            add[8 * (size_t)n + i]);
 }
 
 __device__ FacFluxView flux_view(const FacCoeffs *fc, const double *add, int n, int i, double nu)
@@ -188,12 +190,50 @@ struct OdeShared {
     double v[32], lv[32], vp2[10][32], E1[32], sum[kOdeWarps][32];
 };
 
+// e^{-m x} by rounded products, as flux_sum forms them, for either kernel below: flux_m
+// would otherwise contract the last product with its 1 - e^{-m x}, or not, by what
+// else the kernel takes from it.
+struct OdeExp {
+    double e1, e2, e3, e4, e6;
+    __device__ __forceinline__ explicit OdeExp(double E1)
+    {
+        e1 = E1;
+        e2 = __dmul_rn(e1, e1);
+        e3 = __dmul_rn(e2, e1);
+        e4 = __dmul_rn(e2, e2);
+        e6 = __dmul_rn(e3, e3);
+    }
+    template <int m>
+    __device__ __forceinline__ double of() const
+    {
+        return m == 1 ? e1 : m == 2 ? e2 : m == 3 ? e3 : m == 4 ? e4 : m == 5 ? __dmul_rn(e4, e1) : m == 6 ? e6
+             : m == 7 ? __dmul_rn(e6, e1) : __dmul_rn(e4, e4);
+    }
+};
+
+__device__ __forceinline__ FluxShared ode_flux_shared(const FacFluxView &t, double omega, double Hreal, double L,
+                                                      double v, double lv)
+{
+    FluxShared s;
+    s.omega = omega;
+    s.v = v;
+    s.lv = lv;
+    s.Se = fma(Hreal * Hreal - 1.0, t.c_inv2eta(), 1.0);
+    s.Sodd = v * L;
+    const double v2 = v * v, v4 = v2 * v2;
+    s.v12 = v4 * v4 * v4;
+    s.S2e = s.Se * s.Se;
+    s.S2o = s.Sodd * s.Sodd;
+    s.x = 4.0 * kPi * Hreal * omega;
+    return s;
+}
+
 // the fields of one group of terms, from a full (mostly unused) build
 template <int PART>
 __device__ __forceinline__ void ode_ham_part(OdeShared &sh, const double *add, int n, int i, int lane)
 {
     HamCoeffs h;
-    ham_of_add(&h, add, n, i);
+    ham_of_add<true>(&h, add, n, i);
     auto put = [&](const double &f) {
         sh.ham[(int)(&f - reinterpret_cast<const double *>(&h))][lane] = f;
     };
@@ -290,31 +330,22 @@ __global__ void __cluster_dims__(kOdeWarps, 1, 1) __launch_bounds__(32) k_ctx_od
     cluster.sync();
     const FacFluxView t = flux_view(&ctx[idx ? idx[i] : i], add, n, i, sh.ham[1][lane]);
     {
-        FluxShared s;
-        s.omega = omega;
-        s.v = sh.v[lane];
-        s.lv = sh.lv[lane];
-        s.Se = fma(Hreal * Hreal - 1.0, t.c_inv2eta(), 1.0);
-        s.Sodd = s.v * L;
-        const double v2 = s.v * s.v, v4 = v2 * v2;
-        s.v12 = v4 * v4 * v4;
-        s.S2e = s.Se * s.Se;
-        s.S2o = s.Sodd * s.Sodd;
-        s.x = 4.0 * kPi * Hreal * omega;
+        const FluxShared s = ode_flux_shared(t, omega, Hreal, L, sh.v[lane], sh.lv[lane]);
         double vp2[10];
 #pragma unroll
         for (int q = 0; q < 10; ++q) vp2[q] = sh.vp2[q][lane];
-        const double hw = Hreal * omega, E1 = sh.E1[lane], E2 = E1 * E1, E4 = E2 * E2;
+        const double hw = Hreal * omega;
+        const OdeExp E(sh.E1[lane]);
         double f;
         switch (w) {
-            case 0: f = flux_m<1>(t, s, E1, hw, vp2); break;
-            case 1: f = flux_m<2>(t, s, E2, hw, vp2); break;
-            case 2: f = flux_m<3>(t, s, E2 * E1, hw, vp2); break;
-            case 3: f = flux_m<4>(t, s, E4, hw, vp2); break;
-            case 4: f = flux_m<5>(t, s, E4 * E1, hw, vp2); break;
-            case 5: f = flux_m<6>(t, s, E4 * E2, hw, vp2); break;
-            case 6: f = flux_m<7>(t, s, E4 * (E2 * E1), hw, vp2); break;
-            default: f = flux_m<8>(t, s, E4 * E4, hw, vp2); break;
+            case 0: f = flux_m<1>(t, s, E.of<1>(), hw, vp2); break;
+            case 1: f = flux_m<2>(t, s, E.of<2>(), hw, vp2); break;
+            case 2: f = flux_m<3>(t, s, E.of<3>(), hw, vp2); break;
+            case 3: f = flux_m<4>(t, s, E.of<4>(), hw, vp2); break;
+            case 4: f = flux_m<5>(t, s, E.of<5>(), hw, vp2); break;
+            case 5: f = flux_m<6>(t, s, E.of<6>(), hw, vp2); break;
+            case 6: f = flux_m<7>(t, s, E.of<7>(), hw, vp2); break;
+            default: f = flux_m<8>(t, s, E.of<8>(), hw, vp2); break;
         }
         sh.sum[w][lane] = f;
     }
@@ -330,21 +361,49 @@ __global__ void __cluster_dims__(kOdeWarps, 1, 1) __launch_bounds__(32) k_ctx_od
     k[3 * (size_t)n + i] = -fo;
 }
 
-// The same with one thread per system, for batches that fill the device:
-// a cluster's eight warps repeat what the groups share, so beyond about 32 systems per
-// SM the one chain per thread is the faster (4096 systems: 71 us in clusters, 110 us
-// here; 8192: 111 and 110 us; 16384: 228 and 123 us).
-constexpr int kOdeSystemsPerSm = 32;
+// The same with one thread per system, for batches that fill the device: a cluster's
+// eight warps repeat what the groups share.  GB300, clusters / one thread a system:
+// 4096 systems 71 / 109 us, 7000 105 / 109, 8000 110 / 109, 16384 228 / 119; they cross
+// at 51 systems per SM.  Both give the same bits: the sums and products whose
+// contraction depends on what else a kernel uses of them are written out (FIXED, mul_rn, add_rn).
+// Left to the compiler, 1 system in 4 differed in its last bit, which a free-running
+// integration amplifies, and this kernel took 107 us.
+constexpr int kOdeSystemsPerSm = 48;
 
 __global__ void k_ctx_ode_wide(const FacCoeffs *ctx, const double *arg, double *k, const double *add, int n,
                                const int *idx)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double y[4] = {arg[i], arg[(size_t)n + i], arg[2 * (size_t)n + i], arg[3 * (size_t)n + i]};
-    double kk[4];
-    rhs_ref(ctx, add, n, i, idx ? idx[i] : i, y, kk);
-    for (int q = 0; q < 4; ++q) k[(size_t)q * n + i] = kk[q];
+    const double r = arg[i], pr = arg[2 * (size_t)n + i], L = arg[3 * (size_t)n + i];
+    HamCoeffs h;
+    ham_of_add<true>(&h, add, n, i);
+    HamEval e;
+    ham_eval(h, r, pr, L, &e);
+    const double omega = e.dHdL, Hreal = e.Hreal;
+    const double ro = eob_rcbrt(omega), v = omega * (ro * ro);
+    const double rc = eob_rcbrt(e.omega_c), vphi = omega * (rc * rc), p = vphi * vphi;
+    double vp2[10] = {1.0};
+#pragma unroll
+    for (int j = 1; j < 10; ++j) vp2[j] = vp2[j - 1] * p;
+    const OdeExp E(exp(-4.0 * kPi * Hreal * omega));
+    const double hw = Hreal * omega;
+    const FacFluxView t = flux_view(&ctx[idx ? idx[i] : i], add, n, i, h.nu);
+    const FluxShared s = ode_flux_shared(t, omega, Hreal, L, v, eob_log(v));
+    // each m's last product rounded before the sum, as through shared memory above
+    double sum = flux_m<1>(t, s, E.of<1>(), hw, vp2);
+    sum = __dadd_rn(sum, flux_m<2>(t, s, E.of<2>(), hw, vp2));
+    sum = __dadd_rn(sum, flux_m<3>(t, s, E.of<3>(), hw, vp2));
+    sum = __dadd_rn(sum, flux_m<4>(t, s, E.of<4>(), hw, vp2));
+    sum = __dadd_rn(sum, flux_m<5>(t, s, E.of<5>(), hw, vp2));
+    sum = __dadd_rn(sum, flux_m<6>(t, s, E.of<6>(), hw, vp2));
+    sum = __dadd_rn(sum, flux_m<7>(t, s, E.of<7>(), hw, vp2));
+    sum = __dadd_rn(sum, flux_m<8>(t, s, E.of<8>(), hw, vp2));
+    const double fo = flux_over_omega(t, sum, omega);
+    k[i] = e.dHdpr;
+    k[(size_t)n + i] = omega;
+    k[2 * (size_t)n + i] = -fma(pr * eob_rcp(L), fo, e.dHdr);
+    k[3 * (size_t)n + i] = -fo;
 }
 
 __global__ void k_ctx_rr_force(const FacCoeffs *ctx, double *force, double *g, const double *args, const double *add,

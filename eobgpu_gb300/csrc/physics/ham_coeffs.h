@@ -54,8 +54,31 @@ struct HamCoeffs {
     } d;
 };
 
+// Sums and products that are not contracted beyond what is written.  Host: plain.
+EOB_HD double add_rn(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    return __dadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+
+EOB_HD double mul_rn(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+
 // m_1, m_2 as stored in the reference's additionalArgs (scaled to M = 1 by
-// the waveform class, but any total mass works).
+// the waveform class, but any total mass works).  FIXED writes out the contractions that
+// the compiler would choose by what else a kernel takes from the build: kernels that build a
+// part of the coefficients, or use them without storing them, then agree to the last bit.
+// The set-up's own tables keep the compiler's choice.
+template <bool FIXED = false>
 EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1, double chi_2, double K, double d5,
                              double dSO, double dSS)
 {
@@ -68,13 +91,14 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
     const double c1 = chi_1, c2 = chi_2;
     const double n2 = nu * nu, n3 = n2 * nu, n4 = n3 * nu, n5 = n4 * nu;
     const double s11 = c1 * c1 * X1 * X1, s22 = c2 * c2 * X2 * X2, s12 = c1 * c2 * nu;
-    const double ap2 = s11 + 2.0 * s12 + s22;
+    const double ap2 = FIXED ? add_rn(add_rn(s11, 2.0 * s12), s22) : s11 + 2.0 * s12 + s22;
     const double Kn = K * nu;
     const double K2 = K * K, K4 = K2 * K2, K5 = K4 * K;
     h->M = M;
     h->nu = nu;
     h->ap2 = ap2;
-    h->apsq = (c1 * X1 + c2 * X2) * (c1 * X1 + c2 * X2);
+    const double cX = FIXED ? add_rn(c1 * X1, c2 * X2) : c1 * X1 + c2 * X2;
+    h->apsq = cX * cX;
 
     // ---- AK0 (src/EOB.cu:70)
     for (int k = 0; k < 7; ++k) { h->ak0[k] = 0.0; h->ak0l[k] = 0.0; h->aka[k] = 0.0; }
@@ -135,8 +159,9 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
     for (int k = 0; k < 5; ++k) h->q4c[k] = 0.0;
     for (int k = 0; k < 4; ++k) h->q6c[k] = 0.0;
     for (int k = 0; k < 3; ++k) h->q8c[k] = 0.0;
+    const double q12 = FIXED ? fma(10.0, n2, -(9.0 * nu)) : 10.0 * n2 - 9.0 * nu;
     const double qs = -5.0 * s11 * (X2 * (18.0 * nu - 1.0) + nu * (11.0 * nu - 21.0)) / 8.0 -
-                      5.0 * s12 * (10.0 * n2 - 9.0 * nu - 4.0) / 8.0 -
+                      5.0 * s12 * (q12 - 4.0) / 8.0 -
                       5.0 * s22 * (-18.0 * X2 * nu + X2 + 11.0 * n2 - 3.0 * nu - 1.0) / 8.0;
     h->q8c[1] = nu * (-693359375.0 * l5 - 643896.0 + 59326749.0 * l3 + 1516829440.0 * l2) / 3150.0;
     h->q8h = 5994461.0 * pi * nu / 12700800.0;
@@ -166,7 +191,8 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
     const double nus = nu * (c1 + c2);
     const double g32 = s11 * (-4.0 * X2 - 1.0) / 12.0 + s12 * (0.166666666666667 * X2 - 0.583333333333333) +
                        s22 * (2.0 * X2 - 2.0) / 4.0;
-    const double g31 = -0.5 * s11 * X2 + s12 * (-2.0 * X2 - 5.0) / 12.0 + s22 * (4.0 * X2 - 5.0) / 12.0;
+    const double g31a = -0.5 * s11 * X2, g31b = s12 * (-2.0 * X2 - 5.0) / 12.0;
+    const double g31 = (FIXED ? add_rn(g31a, g31b) : g31a + g31b) + s22 * (4.0 * X2 - 5.0) / 12.0;
     const double soc = dSO * (c1 * X1 + c2 * X2) +
                        (X1 - X2) * (c1 * X1 - c2 * X2) *
                            (7.0 * n4 / 512.0 + 31.0 * n3 / 512.0 + n2 * (208493.0 - 5136.0 * pi2) / 4608.0 -
@@ -185,7 +211,7 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
     gS[1][3] = (14400.0 * n4 - 2477700.0 * n3 - 326100.0 * pi2 * n2 + 19813300.0 * n2 - 89579520.0 * nu * l3 -
                 1672575.0 * pi2 * nu - 3993600.0 * eg * nu + 54396338.0 * nu + 83824640.0 * nu * l2) / 19200.0;
     gSl[1][3] = 1996800.0 * nu / 19200.0;
-    gS[2][0] = (35.0 * n2 + 5.0 * nu) / 8.0;
+    gS[2][0] = (FIXED ? fma(35.0, n2, 5.0 * nu) : 35.0 * n2 + 5.0 * nu) / 8.0;
     gS[2][1] = (-771.0 * n3 + 3324.0 * n2 + 781.0 * nu) / 128.0;
     gS[2][2] = (-38520.0 * n4 - 3309615.0 * n3 + 2872170.0 * n2 - 1626767360.0 * nu * l2 + 19954938.0 * nu +
                 1008889344.0 * nu * l3) / 11520.0;
@@ -197,10 +223,10 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
 
     gT[0][0] = 3.0 / 2.0;
     gT[0][1] = 3.0 * (-2.0 * nu - 3.0) / 8.0;
-    gT[0][2] = 3.0 * (-n2 - 52.0 * nu - 9.0) / 16.0;
+    gT[0][2] = 3.0 * ((FIXED ? add_rn(-n2, -(52.0 * nu)) : -n2 - 52.0 * nu) - 9.0) / 16.0;
     gT[0][3] = (-36.0 * n3 + 4266.0 * n2 - 15254.0 * nu + 492.0 * pi2 * nu - 1215.0) / 384.0;
     gTl[0][4] = 24.0 * nu;
-    gT[1][0] = 3.0 * (-6.0 * nu - 5.0) / 8.0;
+    gT[1][0] = 3.0 * (FIXED ? add_rn(-6.0 * nu, -5.0) : -6.0 * nu - 5.0) / 8.0;
     gT[1][1] = 3.0 * (19.0 * n2 - 12.0 * nu + 23.0) / 16.0;
     gT[1][2] = 3.0 * (36.0 * n3 + 1574.0 * n2 - 558.0 * nu - 15.0) / 64.0;
     gT[1][3] = (5130.0 * n4 - 469440.0 * n3 - 59040.0 * pi2 * n2 + 2316030.0 * n2 - 12317184.0 * nu * l3 -
@@ -223,35 +249,36 @@ EOB_HD void ham_coeffs_build(HamCoeffs *h, double m_1, double m_2, double chi_1,
     h->nc[0][2] += c1 * X1 * g31 + c2 * X2 * g32;
     h->nc[0][4] += soc;
     HamCoeffs::Derived &d = h->d;
-    d.ak0l6 = 6.0 * h->ak0l[6];
-    d.ak0l5 = 5.0 * h->ak0l[5];
-    d.ak0h = 6.5 * h->ak0h;
-    d.fa2 = 2.0 * h->fa2;
-    d.as6 = 6.0 * h->as6;
-    d.as5 = 5.0 * h->as5;
-    d.as4 = 4.0 * h->as4;
-    d.dbl5 = 5.0 * h->dbl[5];
-    d.dbl4 = 4.0 * h->dbl[4];
-    d.dbh = 5.5 * h->dbh;
-    d.bs4 = 4.0 * h->bs4;
-    d.bs3 = 3.0 * h->bs3;
-    d.two_ap2 = 2.0 * h->ap2;
-    d.q4c4 = 4.0 * h->q4c[4];
-    d.q4c3 = 3.0 * h->q4c[3];
-    d.q4c2 = 2.0 * h->q4c[2];
-    d.q4h = 4.5 * h->q4h;
-    d.q6h = 3.5 * h->q6h;
-    d.q6c3 = 3.0 * h->q6c[3];
-    d.q6c2 = 2.0 * h->q6c[2];
-    d.q8h = 2.5 * h->q8h;
-    d.q8c2 = 2.0 * h->q8c[2];
-    d.nc02 = 2.0 * h->nc[0][2];
-    d.nc03 = 3.0 * h->nc[0][3];
-    d.nc04 = 4.0 * h->nc[0][4];
-    d.nc12 = 2.0 * h->nc[1][2];
-    d.nc13 = 3.0 * h->nc[1][3];
-    d.four_n4 = 4.0 * h->nc[4][0];
-    d.two_nu = 2.0 * h->nu;
+    auto times = [](double k, double c) { return FIXED ? mul_rn(k, c) : k * c; };
+    d.ak0l6 = times(6.0, h->ak0l[6]);
+    d.ak0l5 = times(5.0, h->ak0l[5]);
+    d.ak0h = times(6.5, h->ak0h);
+    d.fa2 = times(2.0, h->fa2);
+    d.as6 = times(6.0, h->as6);
+    d.as5 = times(5.0, h->as5);
+    d.as4 = times(4.0, h->as4);
+    d.dbl5 = times(5.0, h->dbl[5]);
+    d.dbl4 = times(4.0, h->dbl[4]);
+    d.dbh = times(5.5, h->dbh);
+    d.bs4 = times(4.0, h->bs4);
+    d.bs3 = times(3.0, h->bs3);
+    d.two_ap2 = times(2.0, h->ap2);
+    d.q4c4 = times(4.0, h->q4c[4]);
+    d.q4c3 = times(3.0, h->q4c[3]);
+    d.q4c2 = times(2.0, h->q4c[2]);
+    d.q4h = times(4.5, h->q4h);
+    d.q6h = times(3.5, h->q6h);
+    d.q6c3 = times(3.0, h->q6c[3]);
+    d.q6c2 = times(2.0, h->q6c[2]);
+    d.q8h = times(2.5, h->q8h);
+    d.q8c2 = times(2.0, h->q8c[2]);
+    d.nc02 = times(2.0, h->nc[0][2]);
+    d.nc03 = times(3.0, h->nc[0][3]);
+    d.nc04 = times(4.0, h->nc[0][4]);
+    d.nc12 = times(2.0, h->nc[1][2]);
+    d.nc13 = times(3.0, h->nc[1][3]);
+    d.four_n4 = times(4.0, h->nc[4][0]);
+    d.two_nu = times(2.0, h->nu);
 }
 
 // ---------------------------------------------------------------------------

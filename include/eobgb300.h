@@ -197,7 +197,7 @@ size_t eob_ctx_bytes(int numSys);
 int eob_ctx_update_information(void *ctx, const double *m1, const double *m2, const double *eta, const double *tplspin,
                                const double *chi_S, const double *chi_A, int use_hm, int numSys,
                                cudaStream_t stream);
-/* src/eob.pyx:158 ODE_Ham_align_AD -> src/EOB.cu:3486 */
+/* src/eob.pyx:158 ODE_Ham_align_AD -> src/EOB.cu:3486; a system's derivatives have the same bits in a batch of any size */
 int eob_ctx_ode(const void *ctx, const double *x, const double *arg, double *k, const double *additionalArgs,
                 int numSys, const int *hCoeffs_index, cudaStream_t stream);
 /* src/eob.pyx:147 RR_force -> src/EOB.cu:3385 */
