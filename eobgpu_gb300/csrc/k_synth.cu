@@ -383,10 +383,12 @@ __device__ __forceinline__ float turns_to_radians(unsigned long long u)
     return fmaf(hi, 0x1.921fb6p-14f, fmaf(hi, -0x1.777a5cp-39f, lo * 0x1.921fb6p-34f));
 }
 
-template <bool VEC>
+// PLAIN: vector loads, no negative m.  Anything else a sample has to allow for (an
+// unaligned workspace, signed products) costs 0.5 and 0.7 % of the kernel.
+template <bool PLAIN>
 __device__ __forceinline__ float4 load_f32(const float *p)
 {
-    if constexpr (VEC) return *reinterpret_cast<const float4 *>(p);
+    if constexpr (PLAIN) return *reinterpret_cast<const float4 *>(p);
     else return make_float4(p[0], p[1], p[2], p[3]);
 }
 
@@ -398,7 +400,7 @@ __device__ __forceinline__ float4 load_f32(const float *p)
 // which wrap as the angle does, so every mode's reduction is free (the FP64
 // reduction of each took 5 instructions of the 37 a five-mode sample had; 10 are
 // left: 4096 binaries, five modes, 12 M samples: 0.95 -> 0.36 ms).
-template <bool VEC>
+template <bool PLAIN>
 __device__ __forceinline__ void mixed_sample(const Ws &w, const SynthArgs &sa, size_t Rc, size_t o, double xx,
                                              float *h_re, float *h_im)
 {
@@ -414,12 +416,13 @@ __device__ __forceinline__ void mixed_sample(const Ws &w, const SynthArgs &sa, s
     const float xf = __uint_as_float(__float_as_uint(f32_trunc(xx)) + (((unsigned)__double2loint(xx) >> 28) & 1u));
     float h = 0.0f, hi = 0.0f;
     for (int q = 0; q < sa.K; ++q) {
-        const float4 a = load_f32<VEC>(w.f32 + 4 * ((size_t)(2 * q) * Rc + o));
-        const float4 c = load_f32<VEC>(w.f32 + 4 * ((size_t)(2 * q + 1) * Rc + o));
+        const float4 a = load_f32<PLAIN>(w.f32 + 4 * ((size_t)(2 * q) * Rc + o));
+        const float4 c = load_f32<PLAIN>(w.f32 + 4 * ((size_t)(2 * q + 1) * Rc + o));
         const float re = fmaf(xf, fmaf(xf, fmaf(xf, a.w, a.z), a.y), a.x);
         const float im = fmaf(xf, fmaf(xf, fmaf(xf, c.w, c.z), c.y), c.x);
         float sp, cp;
-        sincosf(turns_to_radians((unsigned)sa.mms[q] * turn), &sp, &cp);
+        const int m = sa.mms[q];
+        sincosf(turns_to_radians(PLAIN ? (unsigned)m * turn : (unsigned long long)(long long)m * turn), &sp, &cp);
         // (re + i im) e^{-i m phi}
         h = fmaf(re, cp, fmaf(im, sp, h));
         hi = fmaf(im, cp, fmaf(-re, sp, hi));
@@ -432,7 +435,7 @@ __device__ __forceinline__ void mixed_sample(const Ws &w, const SynthArgs &sa, s
 // The FP32 copies exist only if the spline build ran with precision 1
 // (workspace flag queue[6]), and the merger-ringdown runs in FP64 only;
 // otherwise the lnL comes out NaN.
-template <bool VEC>
+template <bool PLAIN>
 __global__ void __launch_bounds__(kSynthThreads) k_synth_mixed_lnl(Ws w, SynthArgs sa)
 {
     __shared__ double s_red[kSynthThreads];
@@ -453,7 +456,7 @@ __global__ void __launch_bounds__(kSynthThreads) k_synth_mixed_lnl(Ws w, SynthAr
                 const double t = grid_time(k, g.dT, g.t0, g.tend);
                 const int i = knot_index(g.x, s_range[0], s_range[1], t);
                 float h, hi;
-                mixed_sample<VEC>(w, sa, Rc, g.base + i, t - g.x[i], &h, &hi);
+                mixed_sample<PLAIN>(w, sa, Rc, g.base + i, t - g.x[i], &h, &hi);
                 const float hk = (float)sa.amp * h;
                 const float term = hk * (hk - 2.0f * w.dataf[k]);
                 // Kahan summation
@@ -469,7 +472,7 @@ __global__ void __launch_bounds__(kSynthThreads) k_synth_mixed_lnl(Ws w, SynthAr
 }
 
 // summed strain, zero past each waveform's end (and without the FP32 copies)
-template <bool VEC>
+template <bool PLAIN>
 __global__ void __launch_bounds__(kSynthThreads) k_synth_mixed_strain(Ws w, SynthArgs sa)
 {
     __shared__ int s_range[2];
@@ -488,7 +491,7 @@ __global__ void __launch_bounds__(kSynthThreads) k_synth_mixed_strain(Ws w, Synt
         if (have_f32) {
             const double t = grid_time(k, g.dT, g.t0, g.tend);
             const int i = knot_index(g.x, s_range[0], s_range[1], t);
-            mixed_sample<VEC>(w, sa, Rc, g.base + i, t - g.x[i], &h, &hi);
+            mixed_sample<PLAIN>(w, sa, Rc, g.base + i, t - g.x[i], &h, &hi);
         }
         put_sample(sa, (size_t)b * sa.N + k, (double)h, (double)hi);
     }
@@ -545,9 +548,10 @@ cudaError_t launch_synth(const Ws &w, const RunArgs &a, int mode, double *out, c
     sa.vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? 1 : 0;
     void (*kern)(Ws, SynthArgs) = mode == 0 ? k_synth_lnl : mode == 2 ? k_synth_strain<2> : k_synth_strain<1>;
     if (mixed) {
-        const bool vec = w.f32_vec();
-        if (mode == 0) kern = vec ? k_synth_mixed_lnl<true> : k_synth_mixed_lnl<false>;
-        else kern = vec ? k_synth_mixed_strain<true> : k_synth_mixed_strain<false>;
+        bool plain = w.f32_vec();
+        for (int j = 0; j < a.K; ++j) plain = plain && a.mms[j] >= 0;
+        if (mode == 0) kern = plain ? k_synth_mixed_lnl<true> : k_synth_mixed_lnl<false>;
+        else kern = plain ? k_synth_mixed_strain<true> : k_synth_mixed_strain<false>;
     }
     const int blocks = mode == 0 ? resident_blocks(kern, kSynthThreads) : nsm * 8;
     kern<<<blocks, kSynthThreads, 0, s>>>(w, sa);
