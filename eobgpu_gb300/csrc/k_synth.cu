@@ -405,15 +405,16 @@ __device__ __forceinline__ void mixed_sample(const Ws &w, const SynthArgs &sa, s
                                              float *h_re, float *h_im)
 {
     const double phi = cubic(w.ys, w.cA, w.cB, w.cC, o, xx);
+    // to nearest (ties away): the truncated bits and the next one
+    float xf = __uint_as_float(__float_as_uint(f32_trunc(xx)) + (((unsigned)__double2loint(xx) >> 28) & 1u));
     unsigned long long turn;
     if ((unsigned)(__double2hiint(phi) & 0x7fffffff) < 0x41000000u) {  // |phi| < 2^17
         turn = (unsigned long long)__double_as_longlong(fma(phi, 0.15915494309189533577, 98304.0));
     } else {
         const double u = phi * 0.15915494309189533577;
         turn = (unsigned long long)__double_as_longlong(u - rint(u) + 98304.0);
+        if ((__double2hiint(phi) & 0x7ff00000) == 0x7ff00000) xf = __int_as_float(0x7fffffff);  // no number: NaN
     }
-    // to nearest (ties away): the truncated bits and the next one
-    const float xf = __uint_as_float(__float_as_uint(f32_trunc(xx)) + (((unsigned)__double2loint(xx) >> 28) & 1u));
     float h = 0.0f, hi = 0.0f;
     for (int q = 0; q < sa.K; ++q) {
         const float4 a = load_f32<PLAIN>(w.f32 + 4 * ((size_t)(2 * q) * Rc + o));

@@ -38,3 +38,22 @@ def test_negative_m(prepared):
     finally:
         wl.mms[0] = 2
     np.testing.assert_allclose(mixed, full, rtol=1e-5)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_phases_that_are_no_numbers(prepared, value):
+    """A phase that is no number makes that binary's likelihood NaN, as in FP64, and no other's."""
+    torch, _lib, wl, data = prepared
+    v = wl.views()
+    off = wl._dev_array(v.row_off, 4, torch.int64).cpu().numpy()
+    phase = wl._dev_array(v.spline_y, int(v.rows_capacity), torch.float64)
+    before = _lnl(wl, data)
+    at = int(off[1]) + 5
+    keep = phase[at].item()
+    phase[at] = value
+    try:
+        mixed, full = _lnl(wl, data), _lnl(wl, data, 0)
+    finally:
+        phase[at] = keep
+    assert np.isnan(mixed).tolist() == np.isnan(full).tolist() == [False, True, False]
+    np.testing.assert_array_equal(mixed[[0, 2]], before[[0, 2]])
