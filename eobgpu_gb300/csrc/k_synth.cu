@@ -134,7 +134,7 @@ __device__ __forceinline__ void put_sample(const SynthArgs &sa, size_t i, double
 __device__ __forceinline__ void ringdown_mode(const ImrRec &c, double x, double *hr, double *hi)
 {
     const double z = fma(c.c1f, x, c.c2f);
-    const double th = z < 20.0 ? 1.0 - 2.0 * eob_rcp(1.0 + exp(2.0 * z)) : 1.0;
+    const double th = z >= 20.0 ? 1.0 : 1.0 - 2.0 * eob_rcp(1.0 + exp(2.0 * z));  // NaN stays NaN
     const double A = fma(c.c1c, th, c.c2c);
     const double ph = c.phi_match - c.d1c * eob_log(fma(c.d2f, exp(-c.d1f * x), 1.0) / (1.0 + c.d2f)) - c.om_re * x;
     const double mag = c.eta * A * exp(-c.om_im * x);
