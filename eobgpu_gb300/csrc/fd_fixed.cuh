@@ -10,9 +10,9 @@
 //
 //  * dot_hi: a sum of two 64-bit products' upper halves from six 32-bit ones (the
 //    products of the low halves, below the last place, left out).
-//  * The delay phase is exact: f tau in units of 2^-64 turn is an integer product;
-//    sine and cosine come from fasttrig.h in units of 2^-61, and the next bin of a
-//    thread by a rotation (2^-58 a step).
+//  * The delay phase: df tau, rounded once, as an integer of 128 bits, whose product with
+//    the bin is exact to 2^-64 turn; sine and cosine come from fasttrig.h in units
+//    of 2^-61, and the next bin of a thread by a rotation (2^-58 a step).
 //    A vector's components share an exponent, so a residual of exactly equal
 //    terms is 2^-57 of their size rather than zero.
 //  * The residual becomes a double again with its exponent, so weights, sums,
@@ -37,28 +37,40 @@ __device__ __forceinline__ i64 dot_hi(i64 a, i64 b, i64 c, i64 d)
     return p + (q >> 31);
 }
 
-__device__ __forceinline__ i64 mul_hi(i64 a, i64 b)
-{
-    const int ah = (int)(a >> 32), bh = (int)(b >> 32);
-    const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
-    return (i64)ah * bh + (((i64)ah * bl + (i64)al * bh) >> 31);
-}
+// u cycles per bin (mod 1, |u| < 2^10: turn_ok) in units of 2^-64 turn and, below them,
+// 2^-128: a double down to 2^-75 fits, so that the phase of bin i, i u, is exact to the
+// last 2^-64 turn.  In 2^-64 alone the cut-off rest, times i, was 6.6e-13 rad in bin 2^21 at
+// df = 1/1024, tau = 1 ms.
+struct Turns {
+    u64 hi, lo;
+    // of bin i
+    __device__ __forceinline__ u64 at(int i) const
+    {
+        const unsigned k = (unsigned)i;
+        const u64 p = (u64)k * (unsigned)(lo >> 32) + (((u64)k * (unsigned)lo) >> 32);
+        return (u64)k * hi + (p >> 32);
+    }
+};
 
-// u cycles per bin in units of 2^-64 turn (mod 1): an integer whose multiples
-// are the phases of the bins (turn_ok: |u| < 2^10)
 __device__ __forceinline__ bool turn_ok(double u)
 {
     return (unsigned)(__double2hiint(u) & 0x7fffffff) < 0x40900000u;
 }
 
-__device__ __forceinline__ u64 turn_of(double u)
+__device__ __forceinline__ Turns turn_of(double u)
 {
     const i64 b = __double_as_longlong(u);
     const int e = (int)((b >> 52) & 0x7ff);
     const u64 m = ((u64)b & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
-    const int sh = e - 1023 - 52 + 64;  // u = m 2^(e - 1023 - 52)
-    const u64 t = sh >= 0 ? (sh < 64 ? m << sh : 0ull) : (sh > -64 ? m >> -sh : 0ull);
-    return b < 0 ? 0ull - t : t;
+    const int sh = e - 1023 - 52 + 128;  // |u| = m 2^sh 2^-128; below 86
+    Turns t;
+    t.hi = sh >= 64 ? m << min(sh - 64, 63) : (sh > 11 ? m >> (64 - sh) : 0ull);
+    t.lo = sh >= 64 ? 0ull : (sh >= 0 ? m << sh : (sh > -64 ? m >> -sh : 0ull));
+    if (b < 0) {
+        t.lo = 0ull - t.lo;
+        t.hi = ~t.hi + (t.lo == 0ull ? 1ull : 0ull);
+    }
+    return t;
 }
 
 // (c, s) turned by (rc, rs)
@@ -110,7 +122,7 @@ __device__ __forceinline__ FdData fd_data(double2 d, double S)
 // 2^e, the phase per bin and its rotation over `stride` bins.
 struct FdDetector {
     i64 fp, fx, rs, rc;
-    u64 step;
+    Turns step;
     int e, slow;
 };
 
@@ -123,7 +135,7 @@ __device__ __forceinline__ FdDetector fd_detector(double fp, double fx, double c
     q.fx = fix_of(fx, e, 8);
     q.e = e - 1023 - 60;
     q.step = turn_of(cycles_per_bin);
-    sincos_fix(q.step * (u64)stride, &q.rs, &q.rc);
+    sincos_fix(q.step.at(stride), &q.rs, &q.rc);
     return q;
 }
 

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kFdThreads, NCH <= 3 ? 3 : 2) k_fd_split_lnl(
         if (threadIdx.x < NCH) dets[threadIdx.x] = det[(size_t)threadIdx.x * B + b];
         __syncthreads();
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) sincos_fix((u64)i0 * dets[c].step, &s[c], &co[c]);
+        for (int c = 0; c < NCH; ++c) sincos_fix(dets[c].step.at(i0), &s[c], &co[c]);
         double acc = 0.0;
         for (int q = 0; q < kFdPerThread; ++q) {
             const int i = i0 + q * kFdThreads;

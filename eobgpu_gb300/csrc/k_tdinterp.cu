@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_fd_lnl(double2 *temp_sum, co
             double acc[NCH];
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
-                sincos_fix((u64)i0 * det[g][c].step, &s[c], &co[c]);
+                sincos_fix(det[g][c].step.at(i0), &s[c], &co[c]);
                 acc[c] = 0.0;
             }
 #pragma unroll
