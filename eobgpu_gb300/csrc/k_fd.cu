@@ -151,10 +151,10 @@ __global__ void __launch_bounds__(kFdThreads, NCH <= 3 ? 3 : 2) k_fd_split_lnl(
                 if (q > 0) rotate(&s[c], &co[c], dets[c].rs, dets[c].rc);
                 const FdData d = fixed[(size_t)c * Nf + i];
                 double power;
-                if (h.slow || dets[c].slow || d.slow) {
+                if (fd_slow(h, dets[c], d)) {
                     const size_t k = (size_t)c * B + b;
                     power = fd_power_slow(p, x, 0.5 * Fplus[k], 0.5 * Fcross[k], data[(size_t)c * Nf + i],
-                                          df * i * tshift[k]);
+                                          df * i * tshift[k], dets[c].slow(), s[c], co[c]);
                 } else {
                     power = fd_power(h, dets[c], s[c], co[c], d);
                 }

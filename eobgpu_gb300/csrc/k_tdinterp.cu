@@ -159,10 +159,10 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_fd_lnl(double2 *temp_sum, co
                         const FdDetector &t = det[g][c];
                         if (q > 0) rotate(&s[c], &co[c], t.rs, t.rc);
                         double power;
-                        if (h.slow || t.slow || d[q][c].slow) {
+                        if (fd_slow(h, t, d[q][c])) {
                             const size_t k = (size_t)(first + c) * B + b0 + g;
                             power = fd_power_slow(p, x, Fplus[k], Fcross[k], data[(size_t)(first + c) * N + i],
-                                                  df * i * tshift[k]);
+                                                  df * i * tshift[k], t.slow(), s[c], co[c]);
                         } else {
                             power = fd_power(h, t, s[c], co[c], d[q][c]);
                         }
