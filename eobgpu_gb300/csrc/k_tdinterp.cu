@@ -51,7 +51,9 @@ __device__ __forceinline__ double2 mode_sum(const double *y, const double *c1, c
         hr = fma(re, c, fma(im, s, hr));
         hi = fma(im, c, fma(-re, s, hi));
     };
-    if (K == 1) {  // the phase m phi rounded once, as a single series' caller would
+    // One mode: m phi rounded to a double, as the reference's sincos(m phi), which tests and
+    // callers compare a single series with; several: exact multiples of the integer phase.
+    if (K == 1) {
         eob::eob_sincos(ms[0] * phi, &s, &c);
         add(0);
         return make_double2(hr, hi);

@@ -10,10 +10,11 @@
 // in Tang's log of fastlog.h), and the angle-addition formulas take the remainder
 // |r| <= pi / 2048 with
 //   sin r = r - r^3 / 6 + r^5 / 120,  cos r - 1 = -r^2 / 2 + r^4 / 24
-// in 64-bit integers: within 2^-59.7, then rounded to a double (half an ulp, and
-// 2^-59.7 absolute, of the exact values for |x| < 2^40, tests/test_gpu_sincos.py).
-// Larger, infinite and NaN arguments take the library's sincos.  Host: the
-// library.
+// in 64-bit integers: within 2^-59.6 of the turn's values (2.4 million turns emulated reach
+// 2^-59.69), 2^-59.2 with the turn's own cut-off, then rounded to a double: half an
+// ulp and 2^-59.2 absolute of the exact values for |x| < 2^40 (tests/test_gpu_sincos.py,
+// tests/test_gpu_phase_turns.py).  Larger, infinite and NaN arguments take the library's
+// sincos.  Host: the library.
 #pragma once
 #include "fac_coeffs.h"
 #include "trig_table.h"
