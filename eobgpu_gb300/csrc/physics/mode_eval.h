@@ -21,10 +21,10 @@
 //
 // mode_eval_sums is the evaluation by the sums of log Gamma throughout, for tables of use_hm = 1.  They
 // cancel from ~30 to order one and leave 4e-15 of rounding in the modulus (rms
-// against 40 digits; 1.5e-15 the closed form).  On the rows of the fine pass (0.05 M
-// apart and less) the third differences of the spline amplify rounding by 1e4
-// to 1e8, so that their c3 is rounding: 4e-15 of the modulus are up to 6e-8 of
-// its norm.  k_modes leaves those rows (4 in 10) to the sums, so that the tables
+// against 40 digits; 1.5e-15 the closed form).  On close rows (the fine pass, 0.05 M
+// apart and less, and the end of the main pass) the third differences of the spline amplify
+// rounding by 1e4 to 1e8, so that their c3 is rounding: 4e-15 of the modulus are up to 6e-8 of
+// its norm.  k_modes leaves rows less than 0.2 M from a neighbour (4 in 10) to the sums, so that the tables
 // do not move with the evaluation of the others; a change of one last bit in the
 // sums (an arctangent by its series, logarithms shared by the modes) moves them too.
 // With derotate = true the result is multiplied by e^{i m phi}: the
